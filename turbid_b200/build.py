@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libturbid_gpu.so")
 BUILD_DIR = os.path.join(HERE, "_build")
 
-CU_SOURCES = ["api.cu", "fft.cu", "gemm.cu", "fields.cu", "islice.cu"]
+CU_SOURCES = ["api.cu", "fft.cu", "fft_mr_f32.cu", "fft_mr_f64.cu", "gemm.cu", "fields.cu", "islice.cu"]
 DRIVER_SRC = os.path.join(HERE, "host", "channelflat_gpu.cc")
 DRIVER = os.path.join(HERE, "channelflat_gpu")
 # the reference's solver-layer library (include/solver_channel_flat.h)

@@ -468,7 +468,7 @@ template <typename T>
 static bool bwd_advection(Ctx& x, const double2* const* src, const int* deriv, int ncomp, const T* unl, T* out,
                           double su, double sv, double sw) {
   const int nf = 3 * ncomp;
-  if (nf * x.nz > x.work_planes || !dft_backward_adv_ok<T>(x.td, x.px, x.py, unl, out)) return false;
+  if (nf * x.nz > x.work_planes || !dft_backward_adv_ok<T>(x.td, x.px, unl, out)) return false;
   SpecGather g{};
   for (int f = 0; f < nf; ++f) {
     g.src[f] = src[f];

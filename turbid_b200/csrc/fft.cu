@@ -12,8 +12,10 @@
 // intermediate is row-major [plane][y][kx], so that each pass reads contiguous
 // blocks (the strided side of the reorder is a write, which the L2 merges
 // into full lines before they reach HBM).
-// The 1-D FFTs are mixed-radix Stockham passes in shared memory with
-// twiddles from a table computed once per length on the host.
+// The 1-D FFTs are Stockham passes with twiddles from a table computed once
+// per length on the host: radix 16 for powers of two (here), grouped radices
+// for the other even lengths with prime factors up to 7 (fft_mr_impl.cuh), one
+// pass per radix in shared memory for the rest (here).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -22,6 +24,7 @@
 #include <cuda.h>
 
 #include "fft_dev.cuh"
+#include "fft_mr.cuh"
 
 namespace tg {
 
@@ -141,24 +144,6 @@ __device__ cplx<T>* fft_batch(cplx<T>* b0, cplx<T>* b1, int NB, const PlanArgs& 
     Ns *= R;
   }
   return in;
-}
-
-// Layout of the backward intermediate: [plane][y][kx] for FP32 (the x pass
-// reads contiguous row blocks), [plane][kx][y] for FP64.
-template <typename T> __host__ __device__ constexpr bool bwd_row_major() { return sizeof(T) == 4; }
-
-// Source plane of a gathered backward launch and the derivative to form on load.
-__device__ __forceinline__ const double2* gather_src(const SpecGather& g, int plane, int nz, int M, int& deriv) {
-  const int gp = g.plane0 + plane, f = gp / nz, z = gp - f * nz;
-  deriv = g.deriv[f];
-  return g.src[f] + (size_t)z * M;
-}
-// coefficient m of the loaded plane, differentiated as (0 + i k) * v (the
-// complex product of SpaceStepper::Gradient, src/stepper_space.cc:373-385)
-__device__ __forceinline__ double2 gather_value(const SpecGather& g, int deriv, int m, double2 v) {
-  if (deriv == 0) return v;
-  const double k = deriv == 1 ? g.kx[m] : g.ky[m];
-  return make_double2(0.0 * v.x - k * v.y, 0.0 * v.y + k * v.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -282,15 +267,15 @@ __global__ void __launch_bounds__(256) fwd_y_kernel(TransformDims d, PlanArgs pl
 }
 
 // backward y pass: spec -> work (zero-filled pruned modes, unscaled)
-template <typename T, int LC, bool GATHER>
+template <typename T, bool GATHER>
 __global__ void __launch_bounds__(256) bwd_y_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
                                                     const double2* __restrict__ spec, cplx<T>* __restrict__ work,
                                                     int NB, SpecGather gat) {
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
-  C* b1 = b0 + NB * (LC > 0 ? LC : pl.L);
-  const int L = LC > 0 ? LC : pl.L;  // == ny
+  C* b1 = b0 + NB * pl.L;
+  const int L = pl.L;  // == ny
   const int plane = blockIdx.y;
   const int k0 = blockIdx.x * NB;
   for (int idx = threadIdx.x; idx < NB * L; idx += blockDim.x) b0[idx] = mkc<C>(0, 0);
@@ -306,7 +291,7 @@ __global__ void __launch_bounds__(256) bwd_y_kernel(TransformDims d, PlanArgs pl
     b0[c * L + d.yidx[iy]] = mkc<C>((T)v.x, (T)v.y);
   }
   __syncthreads();
-  C* r = fft_any<T, +1, LC>(b0, b1, NB, pl, tw);
+  C* r = fft_batch<T, +1>(b0, b1, NB, pl, tw);
   C* dst = work + (size_t)plane * d.nxh * d.ny;
   for (int idx = threadIdx.x; idx < NB * L; idx += blockDim.x) {
     if constexpr (bwd_row_major<T>()) {  // [y][kx]
@@ -323,14 +308,14 @@ __global__ void __launch_bounds__(256) bwd_y_kernel(TransformDims d, PlanArgs pl
 
 // backward x pass: work -> phys [plane][y][x]; two rows per
 // complex FFT; the imaginary part of the kx = 0 coefficient is ignored (c2r).
-template <typename T, int LC>
+template <typename T>
 __global__ void __launch_bounds__(256) bwd_x_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
                                                     const cplx<T>* __restrict__ work, T* __restrict__ phys, int NB) {
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
-  C* b1 = b0 + NB * (LC > 0 ? LC : pl.L);
-  const int L = LC > 0 ? LC : pl.L;  // == nx
+  C* b1 = b0 + NB * pl.L;
+  const int L = pl.L;  // == nx
   const int plane = blockIdx.y;
   const int y0 = blockIdx.x * 2 * NB;
   for (int idx = threadIdx.x; idx < NB * L; idx += blockDim.x) b0[idx] = mkc<C>(0, 0);
@@ -353,7 +338,7 @@ __global__ void __launch_bounds__(256) bwd_x_kernel(TransformDims d, PlanArgs pl
     if (k > 0) b0[p * L + (L - k)] = mkc<C>(h1.x + h2.y, -h1.y + h2.x);
   }
   __syncthreads();
-  C* r = fft_any<T, +1, LC>(b0, b1, NB, pl, tw);
+  C* r = fft_batch<T, +1>(b0, b1, NB, pl, tw);
   T* dst = phys + (size_t)plane * d.ny * d.nx;
   for (int idx = threadIdx.x; idx < NB * L; idx += blockDim.x) {
     const int p = idx / L, x = idx - p * L;
@@ -885,12 +870,14 @@ __global__ void __launch_bounds__(NB * L / 16) bx_p2_kernel(TransformDims d, con
 // never written.  grid: (row blocks x ncomp, nz) with the component fastest:
 // the ncomp CTAs of one row block run together, so the velocity rows they
 // share come from DRAM once and from L2 after; unl: the physical velocity.
+// yfirst: the sum starts with v d/dy instead of u d/dx (its rounding).
 // FP32: registers capped for about 640 threads per SM (measured best).
 template <typename T, int L, int NB>
 __global__ void __launch_bounds__(NB * L / 16, sizeof(T) == 4 ? 640 / (NB * L / 16) : 1) bx_adv_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
                                                                const cplx<T>* __restrict__ work,
                                                                const T* __restrict__ unl, T* __restrict__ out,
-                                                               size_t P, int ncomp, double su, double sv, double sw) {
+                                                               size_t P, int ncomp, double su, double sv, double sw,
+                                                               bool yfirst) {
   using C = cplx<T>;
   using PV = P2Vec<T>;
   using R = typename PV::R;
@@ -905,8 +892,9 @@ __global__ void __launch_bounds__(NB * L / 16, sizeof(T) == 4 ? 640 / (NB * L / 
 #pragma unroll
   for (int i = 0; i < IS; ++i) acca[i] = accb[i] = vzero<R>();
 #pragma unroll 1
-  for (int j = 0; j < 3; ++j) {
-    if (j > 0) __syncthreads();   // buf is refilled
+  for (int i3 = 0; i3 < 3; ++i3) {
+    const int j = yfirst && i3 < 2 ? 1 - i3 : i3;   // the order of the sum
+    if (i3 > 0) __syncthreads();   // buf is refilled
     if constexpr (L >= 16 && PV::kBwdRowMajor) {
       bx_first_pass<T, L, NB>(buf, d, work, (3 * c + j) * d.nz + z, y0);
       __syncthreads();
@@ -984,19 +972,19 @@ template <typename T, int LC>
 static void set_smem_all() {
   set_smem(fwd_x_kernel<T, LC>);
   set_smem(fwd_y_kernel<T, LC>);
-  set_smem(bwd_y_kernel<T, LC, false>);
-  set_smem(bwd_y_kernel<T, LC, true>);
-  set_smem(bwd_x_kernel<T, LC>);
+}
+
+template <typename T>
+static void set_smem_general() {
+  set_smem_all<T, 0>();
+  set_smem(bwd_y_kernel<T, false>);
+  set_smem(bwd_y_kernel<T, true>);
+  set_smem(bwd_x_kernel<T>);
 }
 
 void fft_init() {
-#define TG_INIT_L(L)          \
-  set_smem_all<double, L>(); \
-  set_smem_all<float, L>();
-  TG_FFT_LENGTHS(TG_INIT_L)
-#undef TG_INIT_L
-  set_smem_all<double, 0>();
-  set_smem_all<float, 0>();
+  set_smem_general<double>();
+  set_smem_general<float>();
 }
 
 static bool p2_length(int L) { return L >= 8 && L <= 1024 && (L & (L - 1)) == 0; }
@@ -1029,9 +1017,10 @@ static size_t p2_smem() {
 
 template <typename T>
 bool dft_forward_products_ok(const TransformDims& d, const FftPlan& px, const PhysProduct& prod) {
-  if (!p2_length(px.L) || d.nxh != px.L / 3 * 2 / 2 + 1 || prod.nf < 1 || prod.nf > kMaxGather) return false;
+  const bool p2 = p2_length(px.L);
+  if ((!p2 && !mr_length(px.L)) || d.nxh != px.L / 3 * 2 / 2 + 1 || prod.nf < 1 || prod.nf > kMaxGather) return false;
   for (int f = 0; f < prod.nf; ++f)
-    if (!prod.a[f] || !aligned16(prod.a[f]) || (prod.b[f] && !aligned16(prod.b[f]))) return false;
+    if (!prod.a[f] || (p2 && (!aligned16(prod.a[f]) || (prod.b[f] && !aligned16(prod.b[f]))))) return false;
   return true;
 }
 
@@ -1043,13 +1032,13 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
   PhysProduct pp{};
   if (prod) {
     if (!dft_forward_products_ok<T>(d, px, *prod) || planes != prod->nf * d.nz)
-      throw Error{TG_ERR_SHAPE, "RealCplxCube::DftForward > products on load need a power-of-two Nx"};
+      throw Error{TG_ERR_SHAPE, "RealCplxCube::DftForward > products on load need an Nx that is a power of two or even with prime factors up to 7"};
     pp = *prod;
   }
   {
     prof_begin(s, PC_FFT_FX, (double)planes * d.ny * (d.nx * sizeof(T) + d.nxh * sizeof(C)), 0);
     const C* tw = Tw<T>::get(px);
-    if (prod || (p2_length(px.L) && aligned16(phys) && d.nxh == px.L / 3 * 2 / 2 + 1)) {
+    if (p2_length(px.L) && (prod || aligned16(phys)) && d.nxh == px.L / 3 * 2 / 2 + 1) {
 #define TG_CALL(LL)                                                                         \
   {                                                                                         \
     constexpr int NB = P2Elems<T, P2_FX>::value / LL;                                                \
@@ -1061,7 +1050,7 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
   }
       TG_P2_DISPATCH(px.L, TG_CALL)
 #undef TG_CALL
-    } else {
+    } else if (!mr_forward_x<T>(d, px, phys, work, planes, s, prod)) {
       int nb = pick_nb(px.L, sizeof(C));
       size_t sm = 2 * (size_t)nb * px.L * sizeof(C);
       dim3 grid((d.ny + 2 * nb - 1) / (2 * nb), planes);
@@ -1084,7 +1073,7 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
   }
       TG_P2_DISPATCH(py.L, TG_CALL)
 #undef TG_CALL
-    } else {
+    } else if (!mr_forward_y<T>(d, py, work, spec, planes, scale, s)) {
       int nb = pick_nb(py.L, sizeof(C));
       size_t sm = 2 * (size_t)nb * py.L * sizeof(C);
       dim3 grid((d.nxh + nb - 1) / nb, planes);
@@ -1096,41 +1085,47 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
   }
 }
 
+// y pass of the backward transforms (gather: from the fields' own spectral sources)
+template <typename T>
+static void backward_y(const TransformDims& d, const FftPlan& py, const double2* spec, cplx<T>* w, int planes,
+                       cudaStream_t s, const SpecGather* gather) {
+  using C = cplx<T>;
+  SpecGather gat{};
+  if (gather) gat = *gather;
+  prof_begin(s, PC_FFT_BY, (double)planes * ((double)d.nxh * d.ny * sizeof(C) + (double)d.M * sizeof(double2)), 0);
+  const C* tw = Tw<T>::get(py);
+  if (p2_length(py.L) && d.nyc == py.L / 3 * 2) {
+#define TG_CALL(LL)                                                                                           \
+  {                                                                                                           \
+    constexpr int NB = P2Elems<T, P2_BY>::value / LL;                                                         \
+    dim3 grid((d.nxh + NB - 1) / NB, planes);                                                                 \
+    if (gather)                                                                                               \
+      by_p2_kernel<T, LL, NB, true><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
+    else                                                                                                      \
+      by_p2_kernel<T, LL, NB, false><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
+  }
+    TG_P2_DISPATCH(py.L, TG_CALL)
+#undef TG_CALL
+  } else if (!mr_backward_y<T>(d, py, spec, w, planes, s, gather)) {
+    int nb = pick_nb(py.L, sizeof(C));
+    size_t sm = 2 * (size_t)nb * py.L * sizeof(C);
+    dim3 grid((d.nxh + nb - 1) / nb, planes);
+    const PlanArgs pa = plan_args(py);
+    if (gather)
+      bwd_y_kernel<T, true><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
+    else
+      bwd_y_kernel<T, false><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
+  }
+  prof_end(s);
+  TG_LAUNCH_CHECK("bwd_y_kernel");
+}
+
 template <typename T>
 void dft_backward(const TransformDims& d, const FftPlan& px, const FftPlan& py, const double2* spec, T* phys,
                   int planes, void* work, cudaStream_t s, const SpecGather* gather) {
-  SpecGather gat{};
-  if (gather) gat = *gather;
   using C = cplx<T>;
   C* w = reinterpret_cast<C*>(work);
-  {
-    prof_begin(s, PC_FFT_BY, (double)planes * ((double)d.nxh * d.ny * sizeof(C) + (double)d.M * sizeof(double2)), 0);
-    const C* tw = Tw<T>::get(py);
-    if (p2_length(py.L) && d.nyc == py.L / 3 * 2) {
-#define TG_CALL(LL)                                                                       \
-  {                                                                                       \
-    constexpr int NB = P2Elems<T, P2_BY>::value / LL;                                              \
-    dim3 grid((d.nxh + NB - 1) / NB, planes);                                             \
-    if (gather)                                                                                  \
-      by_p2_kernel<T, LL, NB, true><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
-    else                                                                                        \
-      by_p2_kernel<T, LL, NB, false><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
-  }
-      TG_P2_DISPATCH(py.L, TG_CALL)
-#undef TG_CALL
-    } else {
-      int nb = pick_nb(py.L, sizeof(C));
-      size_t sm = 2 * (size_t)nb * py.L * sizeof(C);
-      dim3 grid((d.nxh + nb - 1) / nb, planes);
-      const PlanArgs pa = plan_args(py);
-      if (gather)
-        bwd_y_kernel<T, 0, true><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
-      else
-        bwd_y_kernel<T, 0, false><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
-    }
-    prof_end(s);
-    TG_LAUNCH_CHECK("bwd_y_kernel");
-  }
+  backward_y<T>(d, py, spec, w, planes, s, gather);
   {
     prof_begin(s, PC_FFT_BX, (double)planes * d.ny * (d.nx * sizeof(T) + d.nxh * sizeof(C)), 0);
     const C* tw = Tw<T>::get(px);
@@ -1143,12 +1138,12 @@ void dft_backward(const TransformDims& d, const FftPlan& px, const FftPlan& py, 
   }
       TG_P2_DISPATCH(px.L, TG_CALL)
 #undef TG_CALL
-    } else {
+    } else if (!mr_backward_x<T>(d, px, work, phys, planes, s)) {
       int nb = pick_nb(px.L, sizeof(C));
       size_t sm = 2 * (size_t)nb * px.L * sizeof(C);
       dim3 grid((d.ny + 2 * nb - 1) / (2 * nb), planes);
       const PlanArgs pa = plan_args(px);
-      bwd_x_kernel<T, 0><<<grid, 256, sm, s>>>(d, pa, tw, w, phys, nb);
+      bwd_x_kernel<T><<<grid, 256, sm, s>>>(d, pa, tw, w, phys, nb);
     }
     prof_end(s);
     TG_LAUNCH_CHECK("bwd_x_kernel");
@@ -1159,10 +1154,8 @@ template void dft_forward<double>(const TransformDims&, const FftPlan&, const Ff
                                   void*, cudaStream_t, const PhysProduct*);
 template void dft_forward<float>(const TransformDims&, const FftPlan&, const FftPlan&, const float*, double2*, int,
                                  void*, cudaStream_t, const PhysProduct*);
-template bool dft_backward_adv_ok<double>(const TransformDims&, const FftPlan&, const FftPlan&, const double*,
-                                          const double*);
-template bool dft_backward_adv_ok<float>(const TransformDims&, const FftPlan&, const FftPlan&, const float*,
-                                         const float*);
+template bool dft_backward_adv_ok<double>(const TransformDims&, const FftPlan&, const double*, const double*);
+template bool dft_backward_adv_ok<float>(const TransformDims&, const FftPlan&, const float*, const float*);
 template void dft_backward_adv<double>(const TransformDims&, const FftPlan&, const FftPlan&, const SpecGather&, int,
                                        const double*, double*, double, double, double, void*, cudaStream_t);
 template void dft_backward_adv<float>(const TransformDims&, const FftPlan&, const FftPlan&, const SpecGather&, int,
@@ -1170,34 +1163,21 @@ template void dft_backward_adv<float>(const TransformDims&, const FftPlan&, cons
 template bool dft_forward_products_ok<double>(const TransformDims&, const FftPlan&, const PhysProduct&);
 template bool dft_forward_products_ok<float>(const TransformDims&, const FftPlan&, const PhysProduct&);
 template <typename T>
-bool dft_backward_adv_ok(const TransformDims& d, const FftPlan& px, const FftPlan& py, const T* unl, const T* out) {
-  return p2_length(px.L) && p2_length(py.L) && d.nxh == px.L / 3 * 2 / 2 + 1 && d.nyc == py.L / 3 * 2 &&
-         aligned16(unl) && aligned16(out) && ((size_t)d.nx * d.ny * d.nz * sizeof(T)) % 16 == 0;
+bool dft_backward_adv_ok(const TransformDims& d, const FftPlan& px, const T* unl, const T* out) {
+  if (d.nxh != px.L / 3 * 2 / 2 + 1) return false;
+  if (p2_length(px.L))
+    return aligned16(unl) && aligned16(out) && ((size_t)d.nx * d.ny * d.nz * sizeof(T)) % 16 == 0;
+  return mr_length(px.L);
 }
 
 template <typename T>
 void dft_backward_adv(const TransformDims& d, const FftPlan& px, const FftPlan& py, const SpecGather& grad, int ncomp,
                       const T* unl, T* out, double su, double sv, double sw, void* work, cudaStream_t s) {
   using C = cplx<T>;
-  if (ncomp < 1 || ncomp > 3 || grad.nf != 3 * ncomp || !dft_backward_adv_ok<T>(d, px, py, unl, out))
-    throw Error{TG_ERR_SHAPE, "RealCplxCube::DftBackward > advection on the x pass needs power-of-two Nx, Ny"};
+  if (ncomp < 1 || ncomp > 3 || grad.nf != 3 * ncomp || !dft_backward_adv_ok<T>(d, px, unl, out))
+    throw Error{TG_ERR_SHAPE, "RealCplxCube::DftBackward > advection on the x pass needs an Nx that is a power of two or even with prime factors up to 7"};
   C* w = reinterpret_cast<C*>(work);
-  const int planes = grad.nf * d.nz;
-  {  // y pass of the gradient fields, derivatives formed on load
-    prof_begin(s, PC_FFT_BY, (double)planes * ((double)d.nxh * d.ny * sizeof(C) + (double)d.M * sizeof(double2)), 0);
-    const C* tw = Tw<T>::get(py);
-    SpecGather gat = grad;
-#define TG_CALL(LL)                                                                                         \
-  {                                                                                                         \
-    constexpr int NB = P2Elems<T, P2_BY>::value / LL;                                                       \
-    dim3 grid((d.nxh + NB - 1) / NB, planes);                                                               \
-    by_p2_kernel<T, LL, NB, true><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, nullptr, w, gat); \
-  }
-    TG_P2_DISPATCH(py.L, TG_CALL)
-#undef TG_CALL
-    prof_end(s);
-    TG_LAUNCH_CHECK("by_p2_kernel");
-  }
+  backward_y<T>(d, py, nullptr, w, grad.nf * d.nz, s, &grad);   // derivatives formed on load
   {  // x pass and the advection sums
     const size_t P = (size_t)d.nx * d.ny * d.nz;
     // per component: three gradient intermediates in, one field out; the velocity once
@@ -1209,12 +1189,15 @@ void dft_backward_adv(const TransformDims& d, const FftPlan& px, const FftPlan& 
   {                                                                                                  \
     constexpr int NB = P2Elems<T, P2_BX>::value / LL;                                                \
     dim3 grid((d.ny + 2 * NB - 1) / (2 * NB) * ncomp, d.nz);                                         \
-    bx_adv_p2_kernel<T, LL, NB><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s>>>(d, tw, w, unl, out, P, ncomp, su, sv, sw); \
+    bx_adv_p2_kernel<T, LL, NB><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s>>>(d, tw, w, unl, out, P, ncomp, su, sv, sw, yfirst); \
   }
-    TG_P2_DISPATCH(px.L, TG_CALL)
+    // d/dy first where a pass is not a power of two: u d/dx + v d/dy then rounds
+    // as the separate advection kernel does
+    const bool yfirst = !p2_length(py.L);
+    if (!mr_backward_adv<T>(d, px, work, unl, out, ncomp, su, sv, sw, s)) { TG_P2_DISPATCH(px.L, TG_CALL) }
 #undef TG_CALL
     prof_end(s);
-    TG_LAUNCH_CHECK("bx_adv_p2_kernel");
+    TG_LAUNCH_CHECK("bx_adv_kernel");
   }
 }
 

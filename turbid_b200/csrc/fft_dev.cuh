@@ -194,5 +194,22 @@ __device__ __forceinline__ void last_pass_out(const cplx<T>* buf, const cplx<T>*
 // spectral row iy -> FFT index along y (P3DFFT pruning, reference src/base.cc:228-237)
 __device__ __forceinline__ int y_of(int iy, int ny, int nyc) { return iy < nyc / 2 ? iy : ny - (nyc - iy); }
 
+// Layout of the backward intermediate: [plane][y][kx] for FP32 (the x pass
+// reads contiguous row blocks), [plane][kx][y] for FP64.
+template <typename T> __host__ __device__ constexpr bool bwd_row_major() { return sizeof(T) == 4; }
+
+// Source plane of a gathered backward launch and the derivative to form on load.
+__device__ __forceinline__ const double2* gather_src(const SpecGather& g, int plane, int nz, int M, int& deriv) {
+  const int gp = g.plane0 + plane, f = gp / nz, z = gp - f * nz;
+  deriv = g.deriv[f];
+  return g.src[f] + (size_t)z * M;
+}
+// coefficient m of the loaded plane, differentiated as (0 + i k) * v (the
+// complex product of SpaceStepper::Gradient, src/stepper_space.cc:373-385)
+__device__ __forceinline__ double2 gather_value(const SpecGather& g, int deriv, int m, double2 v) {
+  if (deriv == 0) return v;
+  const double k = deriv == 1 ? g.kx[m] : g.ky[m];
+  return make_double2(0.0 * v.x - k * v.y, 0.0 * v.y + k * v.x);
+}
 
 }  // namespace tg

@@ -125,7 +125,8 @@ template <typename T>
 void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py,
                  const T* phys, double2* spec, int planes, void* work, cudaStream_t s,
                  const PhysProduct* prod = nullptr);
-// whether dft_forward can form these products on load (power-of-two Nx, 16-byte aligned factors)
+// whether dft_forward can form these products on load (Nx a power of two, with
+// 16-byte aligned factors, or an even length with prime factors up to 7)
 template <typename T>
 bool dft_forward_products_ok(const TransformDims& d, const FftPlan& px, const PhysProduct& prod);
 // Sources of a backward transform launch, one per field of nz planes: the
@@ -147,9 +148,10 @@ void dft_backward(const TransformDims& d, const FftPlan& px, const FftPlan& py,
 // Backward transforms of ncomp groups of three gradient fields (gathered
 // spectral sources, grad.nf = 3 ncomp, grad.plane0 = 0), each group reduced on
 // the x pass to out_c = (u+su) d_c/dx + (v+sv) d_c/dy + (w+sw) d_c/dz with the
-// physical velocity unl (3 fields); power-of-two Nx, Ny only (see _ok).
+// physical velocity unl (3 fields); Nx a power of two or an even length with
+// prime factors up to 7 (see _ok).
 template <typename T>
-bool dft_backward_adv_ok(const TransformDims& d, const FftPlan& px, const FftPlan& py, const T* unl, const T* out);
+bool dft_backward_adv_ok(const TransformDims& d, const FftPlan& px, const T* unl, const T* out);
 template <typename T>
 void dft_backward_adv(const TransformDims& d, const FftPlan& px, const FftPlan& py, const SpecGather& grad, int ncomp,
                       const T* unl, T* out, double su, double sv, double sw, void* work, cudaStream_t s);
