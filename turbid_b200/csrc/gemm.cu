@@ -14,8 +14,8 @@
 //
 // Two kernels:
 //   dense: CTA = MT*8 output rows x 128 reals; 8 warps, each all MT m-tiles x
-//          2 n-tiles; MT chosen per Nz so the row tiles cover Nz with little
-//          padding (257 rows = 3 tiles of 88).
+//          2 n-tiles; MT chosen per launch (launch_tiling; 257 rows at
+//          256x256 = 3 tiles of 88).
 //   sym:   operators with A[n-1-i][n-1-j] = s*A[i][j] (s = +1 for D2, -1 for
 //          D1 on the Chebyshev-Gauss-Lobatto grid).  With h = (n-1)/2 and the
 //          folded input  xe[k] = x[k] + x[n-1-k] (k < h), xe[h] = x[h],
@@ -511,6 +511,39 @@ void row_tiling(int rows, int maxmt, int& mt, int& tiles) {
   mt = (need + tiles - 1) / tiles;
 }
 
+// Row tiling of one launch over `rows` rows and `cols` column tiles (128 reals,
+// all components): the tiling whose busiest SM has the least to do.  A CTA
+// works at the FP64 tensor rate of its SM from two CTAs per SM on, so a launch
+// takes the m-tiles of the SM that gets the most CTAs, times a cost per m-tile
+// that falls with the tile height (the input columns are loaded once per CTA):
+// measured 2.8 + 0.9/mt (dense) and 2.9 + 2/mt (folded) us per 257 rows, and
+// about 15 % more where an SM has one CTA alone.  The fewest row tiles, the
+// choice before, left most SMs idle below some 300 column tiles: one component
+// of 128x128x129 20.6 -> 17.5 us dense (9x2 -> 4x5 m-tiles x row tiles) and
+// 16.5 -> 13.4 folded (5x2 -> 2x5), of 32x32x65 13.5 -> 6.2 and 11.8 -> 5.7,
+// of 128x128x257 65.8 -> 46.8 and 42.5 -> 32.7; 256x256x257 keeps 11x3 and 6x3.
+static void launch_tiling(int rows, int maxmt, bool folded, int cols, int& mt, int& tiles) {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = 148;
+    }
+    return n;
+  }();
+  double best = 0.0;
+  for (int p = maxmt, last = 0; p >= 1; --p) {
+    int m = 0, t = 0;
+    row_tiling(rows, p, m, t);
+    if (t == last) continue;
+    last = t;
+    const long long ctas = (long long)t * cols, per_sm = (ctas + sms - 1) / sms;
+    const double cost = (double)per_sm * m * (folded ? 2.9 + 2.0 / m : 2.8 + 0.9 / m) * (per_sm == 1 ? 1.15 : 1.0);
+    if (best == 0.0 || cost < best) best = cost, mt = m, tiles = t;
+  }
+}
+
 // Rows of the padded operator buffers of an n x n operator: enough for every
 // tiling that a preference in [1, kMaxMtDense] (dense kernel, n rows) or
 // [1, kMaxMtSym] (folded kernel, h+1 rows) selects, so that re-tiling a built
@@ -600,8 +633,8 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
   for (int i = 0; i < nprob; ++i) {
     const ZProblem& pr = probs[i];
     const ZOperator& op = *pr.op;
-    if (op.sym != op0.sym || op.mt != op0.mt || op.tiles != op0.tiles || op.n != op0.n ||
-        (op.split == 2) != (op0.split == 2))
+    if (op.sym != op0.sym || op.mt != op0.mt || op.tiles != op0.tiles || op.n != op0.n || op.rows != op0.rows ||
+        op.pref_dense != op0.pref_dense || op.pref_sym != op0.pref_sym || (op.split == 2) != (op0.split == 2))
       throw Error{TG_ERR_ARG, "zgemm > operators of one launch differ in shape"};
     GemmArgs& g = grp[i];
     g.lda = op.lda;
@@ -642,10 +675,14 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
     grp[i] = grp[0];
     grp[i].batch = 0;
   }
+  // a tiling chosen by the autotuner holds for every launch of the operator
+  int mt = op0.mt, tiles = op0.tiles;
+  if ((op0.sym ? op0.pref_sym : op0.pref_dense) == 0)
+    launch_tiling(op0.rows, op0.sym ? kMaxMtSym : kMaxMtDense, op0.sym, (2 * M + 127) / 128 * total, mt, tiles);
   prof_begin(s, PC_GEMM, by, fl, xfl);
   if (op0.sym) {
     const bool split_in = op0.split == 2;
-    dim3 grid(op0.tiles, (2 * M + 127) / 128, total);
+    dim3 grid(tiles, (2 * M + 127) / 128, total);
 #define TG_SYM(MT, NP, SI) zgemm_sym_kernel<MT, NP, SI><<<grid, kThreads, sym_smem<MT>(), s>>>(grp[0], grp[1], grp[2])
 #define TG_CASE(MT)                                              \
   case MT:                                                       \
@@ -654,11 +691,11 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
     else                                                         \
       split_in ? TG_SYM(MT, kMaxGroup, true) : TG_SYM(MT, kMaxGroup, false); \
     break;
-    switch (op0.mt) { TG_MT_SYM_LIST(TG_CASE) default: throw Error{TG_ERR_ARG, "zgemm > bad tiling"}; }
+    switch (mt) { TG_MT_SYM_LIST(TG_CASE) default: throw Error{TG_ERR_ARG, "zgemm > bad tiling"}; }
 #undef TG_CASE
 #undef TG_SYM
   } else {
-    dim3 grid(op0.tiles, (2 * M + 127) / 128, total);
+    dim3 grid(tiles, (2 * M + 127) / 128, total);
 #define TG_CASE(MT)                                                                                       \
   case MT:                                                                                                \
     if (nprob == 1)                                                                                       \
@@ -666,7 +703,7 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
     else                                                                                                  \
       zgemm_dense_kernel<MT, kMaxGroup><<<grid, kThreads, dense_smem<MT>(), s>>>(grp[0], grp[1], grp[2]); \
     break;
-    switch (op0.mt) { TG_MT_LIST(TG_CASE) default: throw Error{TG_ERR_ARG, "zgemm > bad tiling"}; }
+    switch (mt) { TG_MT_LIST(TG_CASE) default: throw Error{TG_ERR_ARG, "zgemm > bad tiling"}; }
 #undef TG_CASE
   }
   prof_end(s);

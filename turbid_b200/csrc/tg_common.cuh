@@ -229,10 +229,10 @@ struct ZOperator {
   // output, plus x[n-1] += quirk * x[0]
   int split = 0;
   double quirk = 0.0;
-  int rows = 0, mt = 0, tiles = 0;       // launch shape of the kernel used
+  int rows = 0, mt = 0, tiles = 0;       // launch shape of the kernel used (preferences set)
   int mt_dense = 0, tiles_dense = 0;
   // row-tile preferences (most m-tiles of 8 rows per CTA) of the dense and
-  // folded kernels; 0 = the built-in maximum
+  // folded kernels; 0 = chosen per launch
   int pref_dense = 0, pref_sym = 0;
   double* A = nullptr;
   double* Ae = nullptr;
