@@ -29,13 +29,14 @@
 // written in the canonical no-swizzle core-matrix order (8 rows x 16 bytes,
 // K chunks 128 bytes apart, 8-row groups 2048 bytes apart) so that each tile
 // is one contiguous bulk copy into shared memory.  The CTA keeps its 128
-// columns' S data tiles in shared memory, walks the operator in chunks of BN
-// rows (double-buffered bulk copies), and one thread issues the MMAs; after
-// each chunk every thread reads its column's S accumulators from tensor memory
-// (thread i = lane i = data column c0 + i) and stores the chunk's rows of its
-// column, coalesced across the warp.  Every wait is bounded: a wait that gives
-// up sets the error flag, the kernel drains what it issued (bounded too),
-// frees its tensor memory and returns.
+// columns' S data tiles in shared memory and walks the operator in chunks of
+// BN rows; one warp issues the bulk copies, one the MMAs, and sixteen read
+// each chunk's accumulators from tensor memory (thread = lane = data column),
+// hand tensor memory back for the next chunk's MMAs once the diagonals are
+// combined, and store the chunk's rows of their columns, coalesced across the
+// warp.  Only the K steps and operator rows in use are copied and multiplied.
+// Every wait is bounded: a wait that gives up sets the error flag, the kernel
+// drains what it issued (bounded too), frees its tensor memory and returns.
 #include <cfloat>
 #include <climits>
 #include <cstdint>
@@ -49,7 +50,9 @@ namespace {
 
 constexpr int KP = 256;                 // interior rows padded to 8 MMA K-steps of 32
 constexpr int BM = 128;                 // data columns per CTA (MMA M, tensor-memory lanes)
-constexpr int kGemmThreads = 512;        // 16 warps: 4 per lane quarter of the accumulators
+constexpr int kEpiWarps = 16;           // epilogue warps of the product: 4 per lane quarter of the accumulators
+constexpr int kGemmThreads = 32 * (kEpiWarps + 2);   // and one warp each for the MMAs and the copies
+constexpr int kHalfX = BM * 128;        // bytes of a K half of a data tile
 constexpr int kTileX = BM * KP;         // bytes of one data tile
 constexpr int kBadExp = INT_MIN;        // column exponent of a column holding NaN or inf
 // A bounded wait polls at most kSpin times, each poll suspending the thread
@@ -107,8 +110,12 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// true once the phase with the given parity has completed; false after kSpin polls
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// true once the phase with the given parity has completed; false after kSpin
+// polls, or once *stop (when given) is set
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const volatile int* stop = nullptr) {
   for (long long i = 0; i < kSpin; ++i) {
     uint32_t done = 0;
     asm volatile(
@@ -119,6 +126,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         : "r"(bar), "r"(parity), "n"(kSuspendNs)
         : "memory");
     if (done) return true;
+    if (stop && *stop) return false;
   }
   return false;
 }
@@ -140,8 +148,10 @@ template <int S>
 constexpr long long kBias = (S <= 1) ? 0 : 64 * (((1ll << (7 * (S - 1))) - 1) / 127);
 
 // ---------------------------------------------------------------------------
-// Data slicing: a CTA of 16 warps slices 32 columns; warp q reads the 16
-// interior rows of K chunk q (rows 16 q + 1 .. 16 q + 16) of its 32 columns
+// Data slicing: a CTA slices 32 columns with one warp per K chunk in use (the
+// interior rows rounded up to whole MMA K-steps: 16 warps for 257 points, 4
+// for 65); warp q reads the 16 interior rows of K chunk q (rows 16 q + 1 ..
+// 16 q + 16) of its 32 columns
 // (lane = column: 256 contiguous bytes per row), keeps them in registers, the
 // column maxima meet in shared memory, and each warp writes the S slices of
 // its K chunk into the column tile's image (16 bytes per column and slice).
@@ -182,7 +192,8 @@ __global__ void __launch_bounds__(kSliceThreads) k_slice_data(const SliceArgs a)
   __syncthreads();
   mx = 0.0;
 #pragma unroll
-  for (int q = 0; q < KP / 16; ++q) mx = max_keep_nan(mx, part_max[q][lane]);
+  for (int q = 0; q < KP / 16; ++q)
+    if (q < (int)(blockDim.x >> 5)) mx = max_keep_nan(mx, part_max[q][lane]);
   int e = 0;
   const bool bad = !(mx <= DBL_MAX);
   if (!bad && mx > 0.0) {
@@ -246,157 +257,239 @@ struct IslArgs {
   int withhold;            // failure-path check: the operator copies are never issued
 };
 
-// One CTA per 128 data columns, 16 warps.  Thread 0 issues the bulk copies
-// and the MMAs; the operator is streamed in half tiles (BN rows x 128 bytes of
-// K, one contiguous block of the swizzled tile) through four buffers, three
-// copies ahead of the MMAs.  After each chunk of BN operator rows all warps
-// read the accumulators: warp w reads tensor-memory lanes 32 (w % 4) .. +31
-// (data columns) and every fourth 8-row group of the chunk starting at w / 4.
+// One CTA per 128 data columns, 18 warps.
+//   copies (warp 17): the data tiles, then the operator in half tiles (the
+//     chunk's rows x 128 bytes of K, one contiguous block of the swizzled
+//     tile), two at a time through two buffers, each refilled as soon as its
+//     MMAs are done;
+//   MMAs (warp 16): the whole warp walks the slice pairs so that descriptors
+//     stay warp-uniform, one elected lane issues; the accumulators of chunk
+//     j + 1 are started when the sixteen epilogue warps have read chunk j's;
+//   epilogue (warps 0-15): warp w reads tensor-memory lanes 32 (w % 4) .. +31
+//     (data columns) and every fourth 8-row group of the chunk from w / 4 on,
+//     combines the diagonals of its (up to three) groups to integers, releases
+//     the accumulators and finishes from registers beside the next MMAs.
+// Bound by the MMAs' operand reads from shared memory (7 KB per 96-row MMA of
+// 48 cycles, 10 KB per 192-row one of 96; about 80-90 bytes a cycle reached).
+// Slicing and product of one component, before (one thread issuing copies and
+// MMAs in turn, 75-80 cycles per MMA to issue and 600 of waits per half tile,
+// the epilogue between the chunks, K always 256) and now: 257 points at
+// 256x256 114 -> 93 us, 193 at 192x192 60 -> 43, 129 at 128x128 38 -> 24, 65
+// at 64x64 23 -> 16.  Where the cycles of a CTA went is from clock64() marks;
+// with a branch per row the epilogue alone took 14000 cycles a chunk, its FP64
+// chains one after the other.
 template <int S>
 __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs args) {
   using Sh = IslShape<S>;
   constexpr int BN = Sh::BN;
   constexpr int kHalf = Sh::kTileA / 2;               // bytes of one half tile
-  constexpr int NBUF = 4;
-  constexpr uint32_t idesc = idesc_i8(BM, BN);
+  constexpr int NBUF = 2;                             // buffers of two half tiles
+  constexpr int kGroups = BN / 32;                    // 8-row groups per epilogue warp
+  static_assert(BN % 32 == 0, "row groups are dealt to the warps of a lane quarter in turn");
   extern __shared__ __align__(16) uint8_t sm_raw[];
   // swizzle atoms need 1024-byte alignment: round the base up (1 KB reserved)
   uint8_t* sm = sm_raw + ((1024 - (smem_u32(sm_raw) & 1023)) & 1023);
   uint8_t* sx = sm;                                   // S data tiles
-  uint8_t* sa = sm + (size_t)S * kTileX;              // four operator half tiles
-  double* s_aux = reinterpret_cast<double*>(sa + NBUF * kHalf);   // a0, an, asc, lam: 4 x kRowsMax
-  __shared__ __align__(8) uint64_t bars[2 + 2 * NBUF];  // data, accumulators, full[4], empty[4]
+  uint8_t* sa = sm + (size_t)S * kTileX;              // two pairs of operator half tiles
+  double* s_aux = reinterpret_cast<double*>(sa + 2 * NBUF * kHalf);   // a0, an, asc, lam: 4 x kRowsMax
+  __shared__ __align__(8) uint64_t bars[4 + 2 * NBUF];  // data, accumulators, read, drained, full[], empty[]
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_err;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ volatile int s_err;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform
   const int tile = blockIdx.x;
   const IslProblem& a = args.p[blockIdx.y];
-  const uint32_t bar_x = smem_u32(&bars[0]), bar_acc = smem_u32(&bars[1]);
-  auto bar_full = [&](int i) { return smem_u32(&bars[2 + i]); };
-  auto bar_empty = [&](int i) { return smem_u32(&bars[2 + NBUF + i]); };
-  const int total = args.nchunks * S * 2;   // (chunk, operator slice, K half) iterations
+  const uint32_t bar_x = smem_u32(&bars[0]), bar_acc = smem_u32(&bars[1]), bar_read = smem_u32(&bars[2]);
+  const uint32_t bar_drain = smem_u32(&bars[3]), bar_full = smem_u32(&bars[4]), bar_empty = bar_full + 8 * NBUF;
+  const int ncol = args.ncol, nz = args.nz, nrow = args.nrow, nchunks = args.nchunks;
+  const int ksteps = (nz - 2 + 31) / 32, nh = (ksteps + 3) / 4;   // K steps and K halves in use
+  // loads of a chunk: the slice pairs (0, 1), (2, 3) of each K half, then the
+  // K halves of the last slice
+  const int nload = (S / 2) * nh + 1;
+  static_assert(S % 2 == 1, "the last slice has no partner");
 
   if (tid == 0) {
     s_err = 0;
-    for (int i = 0; i < 2 + 2 * NBUF; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    for (int i = 0; i < 4 + 2 * NBUF; ++i) mbar_init(smem_u32(&bars[i]), i == 2 ? kEpiWarps : 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
+  if (warp == kEpiWarps) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   // per-row epilogue constants: boundary columns, row scale, eigenvalue
-  const int rows_pad = args.nchunks * BN;
+  const int rows_pad = nchunks * BN;
   for (int r = tid; r < rows_pad; r += kGemmThreads) {
     s_aux[r] = a.a0[r];
     s_aux[Sh::kRowsMax + r] = a.an[r];
     s_aux[2 * Sh::kRowsMax + r] = a.asc[r];
-    s_aux[3 * Sh::kRowsMax + r] = (a.ep.mode == EPI_RSCALE && r < args.nz) ? a.ep.lam[r] : 0.0;
+    s_aux[3 * Sh::kRowsMax + r] = (a.ep.mode == EPI_RSCALE && r < nz) ? a.ep.lam[r] : 0.0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
+  // operator rows of a chunk, in whole MMA N steps
+  auto chunk_rows = [&](int j) { return min(BN, (nrow - j * BN + 15) / 16 * 16); };
 
-  // operator loads issued (load i goes to buffer i % NBUF), so that an early
-  // exit can drain them
-  int issued = 0;
-  auto issue_op_load = [&](int it) {
-    if (args.withhold) return;   // failure-path check: the full-buffer wait will give up
-    const int buf = it % NBUF;
-    // iteration order = chunk-major, slice, K half: the half tiles lie in that order
-    const int8_t* src = a.as + (size_t)it * kHalf;
-    mbar_expect_tx(bar_full(buf), kHalf);
-    bulk_g2s(smem_u32(sa + buf * kHalf), src, kHalf, bar_full(buf));
-    issued = it + 1;
-  };
-  if (tid == 0) {
-    mbar_expect_tx(bar_x, S * kTileX);
-    for (int p = 0; p < S; ++p)
-      bulk_g2s(smem_u32(sx + p * kTileX), a.xs + ((size_t)tile * S + p) * kTileX, kTileX, bar_x);
-    for (int i = 0; i < NBUF - 1 && i < total; ++i) issue_op_load(i);
-    if (!mbar_wait(bar_x, 0)) s_err = 1;
-  }
-
-  // per-thread column constants: this thread's lane quarter and column
-  const int ncol = args.ncol, nz = args.nz;
-  const int quarter = warp & 3, rgrp = warp >> 2;   // rows: 8-row groups rgrp, rgrp + 4, ...
-  const int c = tile * BM + quarter * 32 + lane;
-  const bool valid = c < ncol;
-  const double xb = valid ? a.in[c] : 0.0;
-  const double xt = valid ? a.in[(size_t)(nz - 1) * ncol + c] : 0.0;
-  const int e = valid ? a.xe[tile * BM + quarter * 32 + lane] : 0;
-  const bool bad = e == kBadExp;
-  const double csc = bad ? 0.0 : ldexp(1.0, e);
-  const int m = c >> 1;
-  const bool rscale = a.ep.mode == EPI_RSCALE;
-  const double k2m = (rscale && valid) ? a.ep.k2[m] : 0.0;
-  double* out = a.out;
-
-  int it = 0;
-  for (int j = 0; j < args.nchunks; ++j) {
-    if (tid == 0 && !s_err) {
-      for (int p = 0; p < S && !s_err; ++p) {
-        for (int h = 0; h < 2; ++h, ++it) {
-          const int buf = it % NBUF;
-          if (!mbar_wait(bar_full(buf), (it / NBUF) & 1)) {
-            s_err = 1;
-            ++it;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa_addr = smem_u32(sa + buf * kHalf);
-          for (int q = 0; q < S - p; ++q) {
-            const uint32_t dacc = tmem + (uint32_t)((p + q) * BN);
-            const uint32_t sx_addr = smem_u32(sx + q * kTileX);
-#pragma unroll
-            for (int kl = 0; kl < 4; ++kl) {
-              const uint64_t da = smem_desc(sx_addr, BM, 4 * h + kl);
-              const uint64_t db = smem_desc(sa_addr, BN, kl);
-              const uint32_t acc = (p == 0 && h == 0 && kl == 0) ? 0u : 1u;   // p = 0 opens every diagonal
-              asm volatile(
-                  "{\n\t.reg .pred pd;\n\t"
-                  "setp.ne.b32 pd, %4, 0;\n\t"
-                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, pd;\n\t}" ::"r"(dacc),
-                  "l"(da), "l"(db), "r"(idesc), "r"(acc));
-            }
-          }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              bar_empty(buf)));
-          // refill the buffer of the previous iteration, NBUF - 1 iterations ahead
-          const int next = it + NBUF - 1;
-          if (next < total) {
-            if (it >= 1 && !mbar_wait(bar_empty((it - 1) % NBUF), ((it - 1) / NBUF) & 1)) {
-              s_err = 1;
-              ++it;
+  if (warp == kEpiWarps + 1) {   // ---- copies
+    if (lane == 0) {
+      mbar_expect_tx(bar_x, S * nh * kHalfX);
+      for (int p = 0; p < S; ++p)
+        bulk_g2s(smem_u32(sx + p * kTileX), a.xs + ((size_t)tile * S + p) * kTileX, nh * kHalfX, bar_x);
+      int issued = 0;
+      bool ok = true;
+      if (!args.withhold)   // failure-path check: the operator copies are never issued, the MMA warp's wait gives up
+        for (int j = 0; j < nchunks && ok; ++j) {
+          const uint32_t bytes = chunk_rows(j) * 128;
+          for (int l = 0; l < nload; ++l) {
+            const int buf = issued % NBUF;
+            if (issued >= NBUF && !mbar_wait(bar_empty + 8 * buf, (issued / NBUF - 1) & 1, &s_err)) {
+              ok = false;
               break;
             }
-            issue_op_load(next);
+            // two half tiles: slices p, p + 1 of one K half, or the K halves of the last slice
+            const bool last = l == nload - 1;
+            const int p = last ? S - 1 : l / nh * 2, h = last ? 0 : l % nh, n = last ? nh : 2;
+            mbar_expect_tx(bar_full + 8 * buf, n * bytes);
+            for (int i = 0; i < n; ++i)
+              bulk_g2s(smem_u32(sa + (2 * buf + i) * kHalf),
+                       a.as + (last ? (size_t)(j * S + p) * 2 + i : (size_t)(j * S + p + i) * 2 + h) * kHalf, bytes,
+                       bar_full + 8 * buf);
+            ++issued;
           }
         }
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_acc));
+      if (!ok) s_err = 1;
+      // every copy issued must have landed before the shared memory is released
+      mbar_wait(bar_x, 0);
+      for (int k = 0; k < NBUF && k < issued; ++k)
+        mbar_wait(bar_full + 8 * k, ((issued - 1 - k) / NBUF) & 1);
     }
-    // every thread: the chunk's accumulators are complete
-    bool ok = mbar_wait(bar_acc, j & 1);
-    ok = __all_sync(0xffffffffu, ok);   // warp-uniform: the tensor-memory loads below are .sync.aligned
-    if (!ok) s_err = 1;
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    if (ok) {
-      const int r0 = j * BN;
+  } else if (warp == kEpiWarps) {   // ---- MMAs
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    const uint64_t dx0 = smem_desc(smem_u32(sx), BM, 0), da0 = smem_desc(smem_u32(sa), BN, 0);
+    bool ok = __all_sync(0xffffffffu, mbar_wait(bar_x, 0, &s_err));
+    auto mma = [&](uint32_t dacc, uint64_t dx, uint64_t db, uint32_t idesc, uint32_t acc) {
+      asm volatile(
+          "{\n\t.reg .pred pd, pe;\n\t"
+          "setp.ne.b32 pd, %4, 0;\n\t"
+          "setp.ne.b32 pe, %5, 0;\n\t"
+          "@pe tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, pd;\n\t}" ::"r"(dacc),
+          "l"(dx), "l"(db), "r"(idesc), "r"(acc), "r"(elected));
+    };
+    int it = 0;
+    for (int j = 0; j < nchunks && ok; ++j) {
+      if (j > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_read, (j - 1) & 1, &s_err));
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int rows = chunk_rows(j);
+      const uint32_t id1 = idesc_i8(BM, rows), id2 = idesc_i8(BM, 2 * BN);
+      for (int l = 0; l < nload && ok; ++l, ++it) {
+        const int buf = it % NBUF;
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * buf, (it / NBUF) & 1, &s_err));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const bool last = l == nload - 1;
+        const int p = last ? S - 1 : l / nh * 2, h0 = last ? 0 : l % nh;
+        const uint64_t db = da0 + (uint64_t)(2 * buf * (kHalf / 16));
+        if (last) {   // slice S-1 with data slice 0
+          for (int kk = 0; kk < ksteps; ++kk)
+            mma(tmem + (uint32_t)((S - 1) * BN), dx0 + (uint64_t)((kk >> 2) * (kHalfX / 16) + 2 * (kk & 3)),
+                db + (uint64_t)((kk >> 2) * (kHalf / 16) + 2 * (kk & 3)), id1, 1u);
+        } else {
+          const int kn = min(4, ksteps - 4 * h0);
 #pragma unroll 1
-      for (int jg = rgrp * 8; jg < BN; jg += 32) {
+          for (int kl = 0; kl < kn; ++kl) {
+            const bool open = p == 0 && h0 == 0 && kl == 0;   // slice 0's first K step opens every diagonal
+            // the pair's products with data slice q lie in adjacent diagonals
+            // p + q, p + q + 1: one MMA of both slices' rows reads the data
+            // tile once, except where slice p opens a diagonal alone or the
+            // chunk has few rows
+            const bool pair = !open && rows > 64;
+            for (int q = 0; q < S - p; ++q) {
+              const uint64_t dx = dx0 + (uint64_t)((q * kTileX + h0 * kHalfX) / 16 + 2 * kl);
+              const uint32_t dacc = tmem + (uint32_t)((p + q) * BN);
+              if (pair && q < S - p - 1)
+                mma(dacc, dx, db + 2u * kl, id2, 1u);
+              else
+                mma(dacc, dx, db + 2u * kl, id1, open ? 0u : 1u);
+            }
+            if (!pair)
+              for (int q = 0; q < S - p - 1; ++q)
+                mma(tmem + (uint32_t)((p + 1 + q) * BN), dx0 + (uint64_t)((q * kTileX + h0 * kHalfX) / 16 + 2 * kl),
+                    db + (uint64_t)(kHalf / 16 + 2 * kl), id1, 1u);
+          }
+        }
+        asm volatile(
+            "{\n\t.reg .pred pe;\n\tsetp.ne.b32 pe, %1, 0;\n\t"
+            "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+                bar_empty + 8 * buf),
+            "r"(elected));
+      }
+      asm volatile(
+          "{\n\t.reg .pred pe;\n\tsetp.ne.b32 pe, %1, 0;\n\t"
+          "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+              ok ? bar_acc : bar_drain),
+          "r"(elected));
+    }
+    if (!ok) {   // the MMAs issued end before tensor and shared memory are released
+      s_err = 1;
+      if (it > 0) mbar_wait(bar_drain, 0);
+    }
+  } else {   // ---- epilogue
+    const int quarter = warp & 3, rgrp = warp >> 2;   // rows: 8-row groups rgrp, rgrp + 4, ...
+    const int c = tile * BM + quarter * 32 + lane;
+    const bool valid = c < ncol;
+    const double xb = valid ? a.in[c] : 0.0;
+    const double xt = valid ? a.in[(size_t)(nz - 1) * ncol + c] : 0.0;
+    const int e = valid ? a.xe[tile * BM + quarter * 32 + lane] : 0;
+    const bool bad = e == kBadExp;
+    const double csc = bad ? 0.0 : ldexp(1.0, e);
+    const int m = c >> 1;
+    const bool rscale = a.ep.mode == EPI_RSCALE;
+    const double k2m = (rscale && valid) ? a.ep.k2[m] : 0.0;
+    double* out = a.out;
+    for (int j = 0; j < nchunks; ++j) {
+      bool ok = mbar_wait(bar_acc, j & 1, &s_err);
+      ok = __all_sync(0xffffffffu, ok);   // warp-uniform: the tensor-memory loads below are .sync.aligned
+      if (!ok) {
+        s_err = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const int r0 = j * BN + rgrp * 8;   // this warp's rows: r0 + 32 g + 0 .. 7
+      // sum_d D_d 2^-(12+7d) = 2^-(12+7(S-1)) sum_d D_d 2^(7(S-1-d)): an
+      // integer below 2^53 in magnitude (|D_d| <= (d+1) 2^20), so the int64
+      // sum and its conversion to FP64 are exact
+      long long isum[kGroups][8];
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        if (r0 + 32 * g >= nrow) continue;
         // the S diagonals' accumulators of 8 rows, all loads in flight before one wait
         uint32_t v[S][8];
 #pragma unroll
         for (int d = 0; d < S; ++d) {
-          const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(d * BN + jg);
+          const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(d * BN + rgrp * 8 + 32 * g);
           asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                        : "=r"(v[d][0]), "=r"(v[d][1]), "=r"(v[d][2]), "=r"(v[d][3]), "=r"(v[d][4]), "=r"(v[d][5]),
                          "=r"(v[d][6]), "=r"(v[d][7])
                        : "r"(taddr));
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          long long u = (int)v[0][i];
+#pragma unroll
+          for (int d = 1; d < S; ++d) u = u * 128 + (int)v[d][i];
+          isum[g][i] = u;
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      if (lane == 0) mbar_arrive(bar_read);   // the next chunk's MMAs may overwrite the accumulators
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        const int rg = r0 + 32 * g;
+        if (rg >= nrow) continue;
         // RSCALE: the reciprocal of a row pair is computed once per mode, the
         // even lane of a (re, im) lane pair taking the first row and the odd
         // lane the second, and exchanged
@@ -404,7 +497,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs a
         if (rscale) {
 #pragma unroll
           for (int i = 0; i < 8; i += 2) {
-            const int rm = r0 + jg + i + (lane & 1);
+            const int rm = rg + i + (lane & 1);
             double R = 1.0;
             if (rm != 0 && rm < nz - 1) {
               const double lam = s_aux[3 * Sh::kRowsMax + rm];
@@ -416,45 +509,35 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs a
             Rpair[i + 1] = (lane & 1) ? R : Ro;
           }
         }
-        if (valid) {
+        // the eight rows' chains of FP64 operations side by side, no branch
+        // between them (rows beyond the last hold zero constants)
+        double val[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int r = r0 + jg + i;
-            // sum_d D_d 2^-(12+7d) = 2^-(12+7(S-1)) sum_d D_d 2^(7(S-1-d)): an
-            // integer below 2^53 in magnitude (|D_d| <= (d+1) 2^20), so the
-            // int64 sum and its conversion to FP64 are exact
-            long long isum = (int)v[0][i];
-#pragma unroll
-            for (int d = 1; d < S; ++d) isum = isum * 128 + (int)v[d][i];
-            const double acc = __ll2double_rn(isum) * (1.0 / (double)(1ll << (12 + 7 * (S - 1))));
-            if (r < args.nrow) {
-              const double interior = __dmul_rn(__dmul_rn(acc, s_aux[2 * Sh::kRowsMax + r]), csc);
-              double val = __dadd_rn(__dadd_rn(__dmul_rn(s_aux[r], xb), interior),
-                                     __dmul_rn(s_aux[Sh::kRowsMax + r], xt));
-              if (bad) val = __longlong_as_double(0x7ff8000000000000LL);
-              if (rscale) val = __dmul_rn(val, Rpair[i]);
-              out[(size_t)r * ncol + c] = val;
-            }
-          }
+        for (int i = 0; i < 8; ++i) {
+          const int r = rg + i;
+          const double acc = __ll2double_rn(isum[g][i]) * (1.0 / (double)(1ll << (12 + 7 * (S - 1))));
+          const double interior = __dmul_rn(__dmul_rn(acc, s_aux[2 * Sh::kRowsMax + r]), csc);
+          val[i] = __dadd_rn(__dadd_rn(__dmul_rn(s_aux[r], xb), interior), __dmul_rn(s_aux[Sh::kRowsMax + r], xt));
+          if (bad) val[i] = __longlong_as_double(0x7ff8000000000000LL);
         }
+        if (rscale) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) val[i] = __dmul_rn(val[i], Rpair[i]);
+        }
+        double* o = out + (size_t)rg * ncol + c;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (valid && rg + i < nrow) o[(size_t)i * ncol] = val[i];
       }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();   // accumulators read before the next chunk's MMAs overwrite them
-    if (s_err) break;  // uniform: read after the barrier
   }
-  // drain: every bulk copy issued must have landed before the shared memory is
-  // released (the MMAs were awaited through the accumulator barrier)
-  if (tid == 0 && s_err) {
-    mbar_wait(bar_x, 0);
-    for (int k = 0; k < NBUF && k < issued; ++k) {
-      const int nk = (issued - 1 - k) / NBUF + 1;   // loads into buffer k
-      mbar_wait(bar_full(k), (nk - 1) & 1);
-    }
-    atomicExch(args.err, 1);
-  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  if (tid == 0 && s_err) atomicExch(args.err, 1);
+  if (warp == kEpiWarps) {
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  }
 }
 
 }  // namespace
@@ -603,7 +686,8 @@ void islice_group(const IsliceOp* const* ops, const double2* const* ins, double2
   const double by = n * (16.0 * M * op0.nz * 2 + (double)op0.ntiles * 5 * kTileX * 2);
   const double fl = n * 4.0 * op0.nz * op0.nz * (double)M;
   prof_begin(s, PC_ISLICE, by, fl, fl);
-  k_slice_data<5><<<dim3(op0.ntiles * (BM / kSliceCols), n), kSliceThreads, 0, s>>>(sa);
+  const int kchunks = (op0.nz - 2 + 31) / 32 * 2;   // 16-row K chunks in use
+  k_slice_data<5><<<dim3(op0.ntiles * (BM / kSliceCols), n), 32 * kchunks, 0, s>>>(sa);
   TG_LAUNCH_CHECK("k_slice_data");
   k_islice_gemm<5><<<dim3(op0.ntiles, n), kGemmThreads, Sh::kSmem, s>>>(a);
   prof_end(s);
