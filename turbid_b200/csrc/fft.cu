@@ -198,7 +198,8 @@ __device__ __forceinline__ cplx<T>* fft_any(cplx<T>* b0, cplx<T>* b1, int NB, co
 // ---------------------------------------------------------------------------
 template <typename T, int LC>
 __global__ void __launch_bounds__(256) fwd_x_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
-                                                    const T* __restrict__ phys, cplx<T>* __restrict__ work, int NB) {
+                                                    const T* phys, cplx<T>* work, int NB) {
+  pdl_begin();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
@@ -239,8 +240,9 @@ __global__ void __launch_bounds__(256) fwd_x_kernel(TransformDims d, PlanArgs pl
 // forward y pass: work [plane][kx][y] -> spec [plane][iy + nyc*kx] (double2)
 template <typename T, int LC>
 __global__ void __launch_bounds__(256) fwd_y_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
-                                                    const cplx<T>* __restrict__ work, double2* __restrict__ spec,
+                                                    const cplx<T>* work, double2* spec,
                                                     int NB, double scale) {
+  pdl_begin();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
@@ -269,8 +271,9 @@ __global__ void __launch_bounds__(256) fwd_y_kernel(TransformDims d, PlanArgs pl
 // backward y pass: spec -> work (zero-filled pruned modes, unscaled)
 template <typename T, bool GATHER>
 __global__ void __launch_bounds__(256) bwd_y_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
-                                                    const double2* __restrict__ spec, cplx<T>* __restrict__ work,
+                                                    const double2* spec, cplx<T>* work,
                                                     int NB, SpecGather gat) {
+  pdl_begin();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
@@ -310,7 +313,8 @@ __global__ void __launch_bounds__(256) bwd_y_kernel(TransformDims d, PlanArgs pl
 // complex FFT; the imaginary part of the kx = 0 coefficient is ignored (c2r).
 template <typename T>
 __global__ void __launch_bounds__(256) bwd_x_kernel(TransformDims d, PlanArgs pl, const cplx<T>* __restrict__ tw,
-                                                    const cplx<T>* __restrict__ work, T* __restrict__ phys, int NB) {
+                                                    const cplx<T>* work, T* phys, int NB) {
+  pdl_begin();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* b0 = reinterpret_cast<C*>(smem_raw);
@@ -387,8 +391,9 @@ template <typename V> __device__ __forceinline__ V vzero() { V v; memset(&v, 0, 
 // forward x pass, L = nx: NB row pairs per CTA, 2 rows packed per complex FFT
 template <typename T, int L, int NB, bool PROD>
 __global__ void __launch_bounds__(NB * L / 16) fx_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
-                                                           const T* __restrict__ phys, cplx<T>* __restrict__ work,
+                                                           const T* phys, cplx<T>* work,
                                                            PhysProduct prod) {
+  pdl_begin();
   using C = cplx<T>;
   using PV = P2Vec<T>;
   using R = typename PV::R;
@@ -517,8 +522,9 @@ __global__ void __launch_bounds__(NB * L / 16) fx_p2_kernel(TransformDims d, con
 // forward y pass, L = ny: NB kx columns per CTA, pruned FP64 output scaled by 1/(Nx*Ny)
 template <typename T, int L, int NB>
 __global__ void __launch_bounds__(NB * L / 16) fy_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
-                                                           const cplx<T>* __restrict__ work,
-                                                           double2* __restrict__ spec, double scale) {
+                                                           const cplx<T>* work,
+                                                           double2* spec, double scale) {
+  pdl_begin();
   using C = cplx<T>;
   using PV = P2Vec<T>;
   using CV = typename PV::CV;
@@ -589,8 +595,9 @@ __global__ void __launch_bounds__(NB * L / 16) fy_p2_kernel(TransformDims d, con
 // backward y pass: zero-filled pruned modes, unscaled
 template <typename T, int L, int NB, bool GATHER>
 __global__ void __launch_bounds__(NB * L / 16) by_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
-                                                           const double2* __restrict__ spec,
-                                                           cplx<T>* __restrict__ work, SpecGather gat) {
+                                                           const double2* spec,
+                                                           cplx<T>* work, SpecGather gat) {
+  pdl_begin();
   using C = cplx<T>;
   constexpr int RS = P2<L>::RS, NT = NB * L / 16;
   constexpr bool RM = P2Vec<T>::kBwdRowMajor;
@@ -704,7 +711,7 @@ __global__ void __launch_bounds__(NB * L / 16) by_p2_kernel(TransformDims d, con
 // threads); the caller synchronises and runs the passes of stride 16 on.
 template <typename T, int L, int NB>
 __device__ __forceinline__ void bx_first_pass(cplx<T>* buf, const TransformDims& d,
-                                              const cplx<T>* __restrict__ work, int plane, int y0) {
+                                              const cplx<T>* work, int plane, int y0) {
   using C = cplx<T>;
   constexpr int RS = P2<L>::RS;
   constexpr int nb = L / 16, nxh = L / 3 * 2 / 2 + 1;
@@ -734,7 +741,7 @@ __device__ __forceinline__ void bx_first_pass(cplx<T>* buf, const TransformDims&
 // Backward x pass, loading half: the zero gap and the row pairs of one work
 // plane combined into the packed two-row FFT input in buf (shared memory).
 template <typename T, int L, int NB>
-__device__ __forceinline__ void bx_fill(cplx<T>* buf, const TransformDims& d, const cplx<T>* __restrict__ work,
+__device__ __forceinline__ void bx_fill(cplx<T>* buf, const TransformDims& d, const cplx<T>* work,
                                         int plane, int y0) {
   using C = cplx<T>;
   using PV = P2Vec<T>;
@@ -809,7 +816,8 @@ __device__ __forceinline__ void bx_fill(cplx<T>* buf, const TransformDims& d, co
 
 template <typename T, int L, int NB>
 __global__ void __launch_bounds__(NB * L / 16) bx_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
-                                                           const cplx<T>* __restrict__ work, T* __restrict__ phys) {
+                                                           const cplx<T>* work, T* phys) {
+  pdl_begin();
   using C = cplx<T>;
   using PV = P2Vec<T>;
   using R = typename PV::R;
@@ -874,10 +882,11 @@ __global__ void __launch_bounds__(NB * L / 16) bx_p2_kernel(TransformDims d, con
 // FP32: registers capped for about 640 threads per SM (measured best).
 template <typename T, int L, int NB>
 __global__ void __launch_bounds__(NB * L / 16, sizeof(T) == 4 ? 640 / (NB * L / 16) : 1) bx_adv_p2_kernel(TransformDims d, const cplx<T>* __restrict__ tw,
-                                                               const cplx<T>* __restrict__ work,
-                                                               const T* __restrict__ unl, T* __restrict__ out,
+                                                               const cplx<T>* work,
+                                                               const T* unl, T* out,
                                                                size_t P, int ncomp, double su, double sv, double sw,
                                                                bool yfirst) {
+  pdl_begin();
   using C = cplx<T>;
   using PV = P2Vec<T>;
   using R = typename PV::R;
@@ -1044,9 +1053,9 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
     constexpr int NB = P2Elems<T, P2_FX>::value / LL;                                                \
     dim3 grid((d.ny + 2 * NB - 1) / (2 * NB), planes);                                      \
     if (prod)                                                                               \
-      fx_p2_kernel<T, LL, NB, true><<<grid, NB * LL / 16, p2_smem<T, LL, P2_FX>(), s>>>(d, tw, phys, w, pp); \
+      launch_pdl(fx_p2_kernel<T, LL, NB, true>, grid, NB * LL / 16, p2_smem<T, LL, P2_FX>(), s, d, tw, phys, w, pp); \
     else                                                                                    \
-      fx_p2_kernel<T, LL, NB, false><<<grid, NB * LL / 16, p2_smem<T, LL, P2_FX>(), s>>>(d, tw, phys, w, pp); \
+      launch_pdl(fx_p2_kernel<T, LL, NB, false>, grid, NB * LL / 16, p2_smem<T, LL, P2_FX>(), s, d, tw, phys, w, pp); \
   }
       TG_P2_DISPATCH(px.L, TG_CALL)
 #undef TG_CALL
@@ -1055,7 +1064,7 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
       size_t sm = 2 * (size_t)nb * px.L * sizeof(C);
       dim3 grid((d.ny + 2 * nb - 1) / (2 * nb), planes);
       const PlanArgs pa = plan_args(px);
-      fwd_x_kernel<T, 0><<<grid, 256, sm, s>>>(d, pa, tw, phys, w, nb);
+      launch_pdl(fwd_x_kernel<T, 0>, grid, 256, sm, s, d, pa, tw, phys, w, nb);
     }
     prof_end(s);
     TG_LAUNCH_CHECK("fwd_x_kernel");
@@ -1069,7 +1078,7 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
   {                                                                                              \
     constexpr int NB = P2Elems<T, P2_FY>::value / LL;                                                     \
     dim3 grid((d.nxh + NB - 1) / NB, planes);                                                    \
-    fy_p2_kernel<T, LL, NB><<<grid, NB * LL / 16, p2_smem<T, LL, P2_FY>(), s>>>(d, tw, w, spec, scale); \
+    launch_pdl(fy_p2_kernel<T, LL, NB>, grid, NB * LL / 16, p2_smem<T, LL, P2_FY>(), s, d, tw, w, spec, scale); \
   }
       TG_P2_DISPATCH(py.L, TG_CALL)
 #undef TG_CALL
@@ -1078,7 +1087,7 @@ void dft_forward(const TransformDims& d, const FftPlan& px, const FftPlan& py, c
       size_t sm = 2 * (size_t)nb * py.L * sizeof(C);
       dim3 grid((d.nxh + nb - 1) / nb, planes);
       const PlanArgs pa = plan_args(py);
-      fwd_y_kernel<T, 0><<<grid, 256, sm, s>>>(d, pa, tw, w, spec, nb, scale);
+      launch_pdl(fwd_y_kernel<T, 0>, grid, 256, sm, s, d, pa, tw, w, spec, nb, scale);
     }
     prof_end(s);
     TG_LAUNCH_CHECK("fwd_y_kernel");
@@ -1100,9 +1109,9 @@ static void backward_y(const TransformDims& d, const FftPlan& py, const double2*
     constexpr int NB = P2Elems<T, P2_BY>::value / LL;                                                         \
     dim3 grid((d.nxh + NB - 1) / NB, planes);                                                                 \
     if (gather)                                                                                               \
-      by_p2_kernel<T, LL, NB, true><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
+      launch_pdl(by_p2_kernel<T, LL, NB, true>, grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s, d, tw, spec, w, gat); \
     else                                                                                                      \
-      by_p2_kernel<T, LL, NB, false><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s>>>(d, tw, spec, w, gat); \
+      launch_pdl(by_p2_kernel<T, LL, NB, false>, grid, NB * LL / 16, p2_smem<T, LL, P2_BY>(), s, d, tw, spec, w, gat); \
   }
     TG_P2_DISPATCH(py.L, TG_CALL)
 #undef TG_CALL
@@ -1112,9 +1121,9 @@ static void backward_y(const TransformDims& d, const FftPlan& py, const double2*
     dim3 grid((d.nxh + nb - 1) / nb, planes);
     const PlanArgs pa = plan_args(py);
     if (gather)
-      bwd_y_kernel<T, true><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
+      launch_pdl(bwd_y_kernel<T, true>, grid, 256, sm, s, d, pa, tw, spec, w, nb, gat);
     else
-      bwd_y_kernel<T, false><<<grid, 256, sm, s>>>(d, pa, tw, spec, w, nb, gat);
+      launch_pdl(bwd_y_kernel<T, false>, grid, 256, sm, s, d, pa, tw, spec, w, nb, gat);
   }
   prof_end(s);
   TG_LAUNCH_CHECK("bwd_y_kernel");
@@ -1134,7 +1143,7 @@ void dft_backward(const TransformDims& d, const FftPlan& px, const FftPlan& py, 
   {                                                                                       \
     constexpr int NB = P2Elems<T, P2_BX>::value / LL;                                              \
     dim3 grid((d.ny + 2 * NB - 1) / (2 * NB), planes);                                    \
-    bx_p2_kernel<T, LL, NB><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s>>>(d, tw, w, phys); \
+    launch_pdl(bx_p2_kernel<T, LL, NB>, grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s, d, tw, w, phys); \
   }
       TG_P2_DISPATCH(px.L, TG_CALL)
 #undef TG_CALL
@@ -1143,7 +1152,7 @@ void dft_backward(const TransformDims& d, const FftPlan& px, const FftPlan& py, 
       size_t sm = 2 * (size_t)nb * px.L * sizeof(C);
       dim3 grid((d.ny + 2 * nb - 1) / (2 * nb), planes);
       const PlanArgs pa = plan_args(px);
-      bwd_x_kernel<T><<<grid, 256, sm, s>>>(d, pa, tw, w, phys, nb);
+      launch_pdl(bwd_x_kernel<T>, grid, 256, sm, s, d, pa, tw, w, phys, nb);
     }
     prof_end(s);
     TG_LAUNCH_CHECK("bwd_x_kernel");
@@ -1189,7 +1198,7 @@ void dft_backward_adv(const TransformDims& d, const FftPlan& px, const FftPlan& 
   {                                                                                                  \
     constexpr int NB = P2Elems<T, P2_BX>::value / LL;                                                \
     dim3 grid((d.ny + 2 * NB - 1) / (2 * NB) * ncomp, d.nz);                                         \
-    bx_adv_p2_kernel<T, LL, NB><<<grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s>>>(d, tw, w, unl, out, P, ncomp, su, sv, sw, yfirst); \
+    launch_pdl(bx_adv_p2_kernel<T, LL, NB>, grid, NB * LL / 16, p2_smem<T, LL, P2_BX>(), s, d, tw, w, unl, out, P, ncomp, su, sv, sw, yfirst); \
   }
     // d/dy first where a pass is not a power of two: u d/dx + v d/dy then rounds
     // as the separate advection kernel does

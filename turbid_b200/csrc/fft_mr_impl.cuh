@@ -244,7 +244,8 @@ __device__ __forceinline__ void mr_last(const cplx<T>* buf, const cplx<T>* __res
 // formed as a[f] (b[f] + shift) (b[f] null: a[f] as it is), planes z-major
 template <typename T, int L>
 __global__ void __launch_bounds__(Mr<L>::NT) mr_fx_kernel(int nz, int ny, const cplx<T>* __restrict__ tw,
-                                                         cplx<T>* __restrict__ work, PhysProduct prod) {
+                                                         cplx<T>* work, PhysProduct prod) {
+  pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr int rows = 2 * P::NB, R = P::R(0), nb = P::nb(0), nxh = L / 3 * 2 / 2 + 1;
@@ -289,8 +290,9 @@ __global__ void __launch_bounds__(Mr<L>::NT) mr_fx_kernel(int nz, int ny, const 
 // forward y pass: kept modes of NB kx columns, FP64, scaled by 1/(Nx*Ny)
 template <typename T, int L>
 __global__ void __launch_bounds__(Mr<L>::NT) mr_fy_kernel(int nxh, const cplx<T>* __restrict__ tw,
-                                                         const cplx<T>* __restrict__ work,
-                                                         double2* __restrict__ spec, double scale) {
+                                                         const cplx<T>* work,
+                                                         double2* spec, double scale) {
+  pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr int R = P::R(0), nb = P::nb(0), nyc = L / 3 * 2, h = nyc / 2;
@@ -318,7 +320,8 @@ __global__ void __launch_bounds__(Mr<L>::NT) mr_fy_kernel(int nxh, const cplx<T>
 // alone: both tables are constant along the other index)
 template <typename T, int L>
 __global__ void __launch_bounds__(Mr<L>::NT) mr_by_kernel(int nz, int nxh, const cplx<T>* __restrict__ tw,
-                                                         cplx<T>* __restrict__ work, SpecGather gat) {
+                                                         cplx<T>* work, SpecGather gat) {
+  pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr bool RM = bwd_row_major<T>();
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(Mr<L>::NT) mr_by_kernel(int nz, int nxh, const
 // conj X[k], zero between the kept bands, Im of kx = 0 ignored (c2r)
 template <typename T, int L>
 __device__ __forceinline__ void mr_bx_first(cplx<T>* buf, const cplx<T>* __restrict__ tw,
-                                            const cplx<T>* __restrict__ src, int ny, int y0) {
+                                            const cplx<T>* src, int ny, int y0) {
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr bool RM = bwd_row_major<T>();
@@ -389,7 +392,8 @@ __device__ __forceinline__ void mr_bx_first(cplx<T>* buf, const cplx<T>* __restr
 
 template <typename T, int L>
 __global__ void __launch_bounds__(Mr<L>::NT) mr_bx_kernel(int ny, const cplx<T>* __restrict__ tw,
-                                                         const cplx<T>* __restrict__ work, T* __restrict__ phys) {
+                                                         const cplx<T>* work, T* phys) {
+  pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr int nxh = L / 3 * 2 / 2 + 1;
@@ -416,9 +420,10 @@ __global__ void __launch_bounds__(Mr<L>::NT) mr_bx_kernel(int ny, const cplx<T>*
 template <typename T, int L>
 __global__ void __launch_bounds__(Mr<L>::NT, sizeof(T) == 4 ? 640 / Mr<L>::NT : 1)
     mr_adv_kernel(int nz, int ny, const cplx<T>* __restrict__ tw,
-                                                          const cplx<T>* __restrict__ work,
-                                                          const T* __restrict__ unl, T* __restrict__ out,
+                                                          const cplx<T>* work,
+                                                          const T* unl, T* out,
                                                           int ncomp, double su, double sv, double sw) {
+  pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
   constexpr int nxh = L / 3 * 2 / 2 + 1;
@@ -496,7 +501,7 @@ bool mr_forward_x(const TransformDims& d, const FftPlan& px, const T* phys, void
   }
   return mr_dispatch(d.nx, [&](auto lc) {
     using P = Mr<decltype(lc)::value>;
-    mr_fx_kernel<T, decltype(lc)::value><<<dim3(blocks(d.ny, 2 * P::NB), planes), P::NT, P::template smem<T>(), s>>>(nz, d.ny, Tw<T>::get(px), reinterpret_cast<cplx<T>*>(work), pp);
+    launch_pdl(mr_fx_kernel<T, decltype(lc)::value>, dim3(blocks(d.ny, 2 * P::NB), planes), P::NT, P::template smem<T>(), s, nz, d.ny, Tw<T>::get(px), reinterpret_cast<cplx<T>*>(work), pp);
   });
 }
 
@@ -505,7 +510,7 @@ bool mr_forward_y(const TransformDims& d, const FftPlan& py, const void* work, d
                   cudaStream_t s) {
   return mr_dispatch(d.ny, [&](auto lc) {
     using P = Mr<decltype(lc)::value>;
-    mr_fy_kernel<T, decltype(lc)::value><<<dim3(blocks(d.nxh, P::NB), planes), P::NT, P::template smem<T>(), s>>>(d.nxh, Tw<T>::get(py), reinterpret_cast<const cplx<T>*>(work), spec, scale);
+    launch_pdl(mr_fy_kernel<T, decltype(lc)::value>, dim3(blocks(d.nxh, P::NB), planes), P::NT, P::template smem<T>(), s, d.nxh, Tw<T>::get(py), reinterpret_cast<const cplx<T>*>(work), spec, scale);
   });
 }
 
@@ -523,7 +528,7 @@ bool mr_backward_y(const TransformDims& d, const FftPlan& py, const double2* spe
   }
   return mr_dispatch(d.ny, [&](auto lc) {
     using P = Mr<decltype(lc)::value>;
-    mr_by_kernel<T, decltype(lc)::value><<<dim3(blocks(d.nxh, P::NB), planes), P::NT, P::template smem<T>(), s>>>(nz, d.nxh, Tw<T>::get(py), reinterpret_cast<cplx<T>*>(work), g);
+    launch_pdl(mr_by_kernel<T, decltype(lc)::value>, dim3(blocks(d.nxh, P::NB), planes), P::NT, P::template smem<T>(), s, nz, d.nxh, Tw<T>::get(py), reinterpret_cast<cplx<T>*>(work), g);
   });
 }
 
@@ -531,7 +536,7 @@ template <typename T>
 bool mr_backward_x(const TransformDims& d, const FftPlan& px, const void* work, T* phys, int planes, cudaStream_t s) {
   return mr_dispatch(d.nx, [&](auto lc) {
     using P = Mr<decltype(lc)::value>;
-    mr_bx_kernel<T, decltype(lc)::value><<<dim3(blocks(d.ny, 2 * P::NB), planes), P::NT, P::template smem<T>(), s>>>(d.ny, Tw<T>::get(px), reinterpret_cast<const cplx<T>*>(work), phys);
+    launch_pdl(mr_bx_kernel<T, decltype(lc)::value>, dim3(blocks(d.ny, 2 * P::NB), planes), P::NT, P::template smem<T>(), s, d.ny, Tw<T>::get(px), reinterpret_cast<const cplx<T>*>(work), phys);
   });
 }
 
@@ -540,7 +545,7 @@ bool mr_backward_adv(const TransformDims& d, const FftPlan& px, const void* work
                      double su, double sv, double sw, cudaStream_t s) {
   return mr_dispatch(d.nx, [&](auto lc) {
     using P = Mr<decltype(lc)::value>;
-    mr_adv_kernel<T, decltype(lc)::value><<<dim3(blocks(d.ny, 2 * P::NB) * ncomp, d.nz), P::NT, P::template smem<T>(), s>>>(d.nz, d.ny, Tw<T>::get(px), reinterpret_cast<const cplx<T>*>(work), unl, out, ncomp, su, sv, sw);
+    launch_pdl(mr_adv_kernel<T, decltype(lc)::value>, dim3(blocks(d.ny, 2 * P::NB) * ncomp, d.nz), P::NT, P::template smem<T>(), s, d.nz, d.ny, Tw<T>::get(px), reinterpret_cast<const cplx<T>*>(work), unl, out, ncomp, su, sv, sw);
   });
 }
 

@@ -22,6 +22,7 @@ __device__ __forceinline__ double2 mul_i(double k, double2 x) {  // (0, k) * x
 
 // --- layout conversion: reference [c][m][z] <-> slab [c][z][m] ---------------
 __global__ void k_ref_to_slab(const double2* __restrict__ ref, double2* __restrict__ slab, int M, int nz) {
+  pdl_begin();
   __shared__ double2 t[32][33];
   const int c = blockIdx.z;
   const double2* src = ref + (size_t)c * M * nz;
@@ -38,6 +39,7 @@ __global__ void k_ref_to_slab(const double2* __restrict__ ref, double2* __restri
   }
 }
 __global__ void k_slab_to_ref(const double2* __restrict__ slab, double2* __restrict__ ref, int M, int nz) {
+  pdl_begin();
   __shared__ double2 t[32][33];
   const int c = blockIdx.z;
   const double2* src = slab + (size_t)c * M * nz;
@@ -69,6 +71,7 @@ void slab_to_ref(const double2* slab, double2* ref, int M, int nz, int dim, cuda
 // distinct ones uu, uv, uw, vv, vw, ww (u_i u_j == u_j u_i exactly).
 template <typename T>
 __global__ void k_products6(const T* __restrict__ unl, T* __restrict__ prd, size_t P) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x) {
     T u = unl[i], v = unl[P + i], w = unl[2 * P + i];
     prd[i] = u * u;
@@ -94,6 +97,7 @@ void products6(const T* unl, T* prd, size_t P, cudaStream_t s) {
 template <typename T>
 __global__ void k_adv(const T* __restrict__ unl, const T* __restrict__ dup, T* __restrict__ out, size_t P, int ncomp,
                       double su, double sv, double sw) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x) {
     T u = unl[i] + (T)su, v = unl[P + i] + (T)sv, w = unl[2 * P + i] + (T)sw;
     for (int c = 0; c < ncomp; ++c) {
@@ -115,6 +119,7 @@ void adv_products(const T* unl, const T* dup, T* out, size_t P, int ncomp, doubl
 template <typename T>
 __global__ void k_phi_products(const T* __restrict__ phip, const T* __restrict__ unl, T* __restrict__ out, size_t P,
                                double su, double sv, double sw) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x) {
     T p = phip[i];
     out[i] = p * (unl[i] + (T)su);
@@ -134,6 +139,7 @@ void phi_products(const T* phip, const T* unl, T* out, size_t P, double su, doub
 template <typename T>
 __global__ void k_mul_shift(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, size_t P,
                             double sh) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < P; i += (size_t)gridDim.x * blockDim.x)
     out[i] = (b[i] + (T)sh) * a[i];
 }
@@ -149,6 +155,7 @@ void mul_shift(const T* a, const T* b, T* out, size_t P, double sh, cudaStream_t
 __global__ void k_h_update(double2* __restrict__ H, const double2* __restrict__ adv, const double2* __restrict__ phi,
                            size_t S, int M, double c1, double dt, double bcoef, double sinsl, double cossl, int sdir,
                            double dtf1, double dtf2, const double* __restrict__ dtf) {
+  pdl_begin();
   const size_t n = 3 * S;
   if (dtf) {  // forcing of this step from device memory (graph replay)
     dtf1 = dtf[0];
@@ -196,6 +203,7 @@ void h_update(double2* H, const double2* adv, const double2* phi, size_t S, int 
 // that produces phi has finished.
 __global__ void k_buoyancy(double2* __restrict__ H, double2* __restrict__ rhs, const double2* __restrict__ phi, int M,
                            int nz, double bcoef, double trig, int sgn, double ac2) {
+  pdl_begin();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   const int z = blockIdx.y;
@@ -232,6 +240,7 @@ void buoyancy(double2* H, double2* rhs, const double2* phi, int M, int nz, doubl
 
 // scalar register (phase_scalar_flat.cc:308-310)
 __global__ void k_axpby(double2* __restrict__ y, const double2* __restrict__ x, size_t n, double a, double b) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double2 v = y[i], w = x[i];
     y[i] = make_double2(a * v.x - b * w.x, a * v.y - b * w.y);
@@ -250,6 +259,7 @@ void axmby(double2* y, const double2* x, size_t n, double a, double b, cudaStrea
 // 0 dp1m1top 1 dp1m1bot 2 dp1m2top 3 dp1m2bot 4 dp2m1top 5 dp2m1bot 6 dp2m2top 7 dp2m2bot
 __global__ void k_boundary_apply(double2* __restrict__ rhs, const double2* __restrict__ hist, size_t S, int M, int nz,
                                  double fac, double r, int opentop, double tu, double tv, double tw) {
+  pdl_begin();
   const int n = 3 * M;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int c = i / M, m = i - c * M;
@@ -330,6 +340,7 @@ __global__ void k_boundary_update(double2* __restrict__ hist, const double2* __r
                                   const double2* __restrict__ dpz, int M, int nz, int opentop,
                                   const double* __restrict__ kx, const double* __restrict__ ky,
                                   const double* __restrict__ d1r0, const double* __restrict__ d1rn) {
+  pdl_begin();
   const size_t R = (size_t)3 * M;
   const int m = blockIdx.x * 32 + threadIdx.x;
   if (threadIdx.y < 3 && m < M) {
@@ -371,6 +382,7 @@ void boundary_update(double2* hist, const double2* p, const double2* dpz, int M,
 // features, phase_carrier_flat.cc:687-692).
 __global__ void k_wall_dz(const double2* __restrict__ U, double2* __restrict__ DU, size_t S, int M, int nz,
                           const double* __restrict__ d1r0, const double* __restrict__ d1rn) {
+  pdl_begin();
   const int c = blockIdx.y;
   const int m = blockIdx.x * 32 + threadIdx.x;
   double2 r0, rn;
@@ -393,6 +405,7 @@ void wall_dz(const double2* U, double2* DU, size_t S, int M, int nz, const doubl
 __global__ void k_project(double2* __restrict__ U, const double2* __restrict__ SU, const double2* __restrict__ P,
                           const double2* __restrict__ DPZ, size_t S, int M, const double* __restrict__ kx,
                           const double* __restrict__ ky, double coef) {
+  pdl_begin();
   const size_t n = 3 * S;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(i / S);
@@ -414,6 +427,7 @@ void project(double2* U, const double2* SU, const double2* P, const double2* DPZ
 
 // rows 0 and N-1 := 0 (boundary_scalar_flat.cc:150-151)
 __global__ void k_zero_rows(double2* f, int M, int nz) {
+  pdl_begin();
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     f[m] = make_double2(0.0, 0.0);
     f[(size_t)(nz - 1) * M + m] = make_double2(0.0, 0.0);
@@ -428,6 +442,7 @@ void zero_rows(double2* f, int M, int nz, cudaStream_t s) {
 template <typename T>
 __global__ void k_erosion_tau(const T* __restrict__ dudz, const T* __restrict__ dvdz, T* __restrict__ tau, size_t n,
                               double re, double tauc, double rate) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     T a = dudz[i], b = dvdz[i];
     T v = sqrt(a * a + b * b) / (T)re;
@@ -443,6 +458,7 @@ void erosion_tau(const T* dudz, const T* dvdz, T* tau, size_t n, double re, doub
 
 __global__ void k_erosion_row(double2* __restrict__ rhs, const double2* __restrict__ ero, const double2* __restrict__ phi,
                               int M, double wsc, double conc, double resc, double* feat) {
+  pdl_begin();
   for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
     double2 e = ero[m], p = phi[m];
     double2 r = make_double2(e.x - wsc * p.x * conc, e.y - wsc * p.y * conc);
@@ -503,7 +519,8 @@ struct alignas(sizeof(T) * W) FilterVec {
 };
 
 template <typename T, int W>
-__global__ void __launch_bounds__(kFilterThreads, 2) k_filter(T* __restrict__ phip, int plane_n) {
+__global__ void __launch_bounds__(kFilterThreads, 2) k_filter(T* phip, int plane_n) {
+  pdl_begin();
   using V = FilterVec<T, W>;
   constexpr int FB = kFilterBatch / W, STEP = FB * kFilterThreads;
   __shared__ double red[4][32];
@@ -565,9 +582,9 @@ void positivity_filter(T* phip, int plane_n, int nz, cudaStream_t s) {
   prof_begin(s, PC_FILTER, 11.0 * sizeof(T) * (double)plane_n * nz, 0);   // 6 reads + 5 writes of the plane
   constexpr int W = 16 / sizeof(T);
   if (plane_n % W == 0 && reinterpret_cast<uintptr_t>(phip) % 16 == 0)
-    k_filter<T, W><<<nz, kFilterThreads, 0, s>>>(phip, plane_n);
+    launch_pdl(k_filter<T, W>, nz, kFilterThreads, 0, s, phip, plane_n);
   else
-    k_filter<T, 1><<<nz, kFilterThreads, 0, s>>>(phip, plane_n);
+    launch_pdl(k_filter<T, 1>, nz, kFilterThreads, 0, s, phip, plane_n);
   prof_end(s);
   TG_LAUNCH_CHECK("k_filter");
 }
@@ -584,6 +601,7 @@ __device__ __forceinline__ double max_keep_nan(double a, double b) { return (b >
 template <typename T>
 __global__ void k_feature_max(const T* __restrict__ unl, int nx, int ny, int nz, const double* __restrict__ glz,
                               double lmx, double lmy, unsigned long long* bits) {
+  pdl_begin();
   // blockIdx.y = z plane: the wall maxima and 1/glz need no per-element index division
   const size_t plane = (size_t)nx * ny, P = plane * nz;
   const int z = blockIdx.y;
@@ -644,6 +662,7 @@ __global__ void k_feature_max(const T* __restrict__ unl, int nx, int ny, int nz,
 // flocal = feat[0..49], fglobal = feat[50..99]
 __global__ void k_feature_final(double* feat, const unsigned long long* bits, const double2* __restrict__ du, size_t S,
                                 int M, int nz) {
+  pdl_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   for (int k = 0; k < 9; ++k) feat[k] = __longlong_as_double((long long)bits[k]);
   feat[19] = __longlong_as_double((long long)bits[9]);
@@ -674,6 +693,7 @@ void features(const T* unl, int nx, int ny, int nz, const double* glz, double lm
 // phase_carrier_flat.cc:509, phase_scalar_flat.cc:485-518)
 __global__ void k_trapz_mean(const double2* __restrict__ f, int M, int nz, const double* __restrict__ gz, double shift,
                              double* feat, int slot) {
+  pdl_begin();
   // one warp: lane-strided intervals, then a shuffle sum
   double s = 0.0;
   for (int k = threadIdx.x; k < nz - 1; k += 32)
@@ -690,6 +710,7 @@ void trapz_mean(const double2* f, int M, int nz, const double* gz, double shift,
 }
 
 __global__ void k_set_feat(double* feat, int slot, double v) {
+  pdl_begin();
   if (threadIdx.x == 0 && blockIdx.x == 0) feat[slot] = v;
 }
 void set_feat(double* feat, int slot, double v, cudaStream_t s) {
@@ -700,6 +721,7 @@ void set_feat(double* feat, int slot, double v, cudaStream_t s) {
 // --- precision conversions for the mixed path --------------------------------------
 template <typename A, typename B>
 __global__ void k_convert(const A* __restrict__ a, B* __restrict__ b, size_t n) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     b[i] = (B)a[i];
 }
@@ -730,6 +752,7 @@ namespace tg {
 // when D = (q/2)^2 + (p/3)^3 > 0, and then (Cardano) the pair is
 // -(u + v)/2 +- i sqrt(3)/2 (u - v) with u = cbrt(-q/2 + sqrt(D)), u v = -p/3.
 __global__ void k_swirling(const double* __restrict__ g, size_t fstride, size_t n, double* __restrict__ out) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     double a[9];
 #pragma unroll

@@ -455,6 +455,7 @@ __device__ __forceinline__ void sym_body(const GemmArgs& g, const int b) {
 
 template <int MT, int NP>
 __global__ void __launch_bounds__(kThreads) zgemm_dense_kernel(GemmArgs g0, GemmArgs g1, GemmArgs g2) {
+  pdl_begin();
 #define TG_BODY(G, Z) dense_body<MT>(G, Z)
   TG_GROUP_DISPATCH(TG_BODY)
 #undef TG_BODY
@@ -462,6 +463,7 @@ __global__ void __launch_bounds__(kThreads) zgemm_dense_kernel(GemmArgs g0, Gemm
 
 template <int MT, int NP, bool SPLIT_IN>
 __global__ void __launch_bounds__(kThreads, 2) zgemm_sym_kernel(GemmArgs g0, GemmArgs g1, GemmArgs g2) {
+  pdl_begin();
 #define TG_BODY(G, Z) sym_body<MT, SPLIT_IN>(G, Z)
   TG_GROUP_DISPATCH(TG_BODY)
 #undef TG_BODY
@@ -511,6 +513,29 @@ void row_tiling(int rows, int maxmt, int& mt, int& tiles) {
   mt = (need + tiles - 1) / tiles;
 }
 
+int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = 148;
+    }
+    return n;
+  }();
+  return sms;
+}
+
+bool early_launch(dim3 grid, cudaStream_t s) {
+  if (2ll * grid.x * grid.y * grid.z > sm_count()) return false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return st == cudaStreamCaptureStatusNone;
+}
+
 // Row tiling of one launch over `rows` rows and `cols` column tiles (128 reals,
 // all components): the tiling whose busiest SM has the least to do.  A CTA
 // works at the FP64 tensor rate of its SM from two CTAs per SM on, so a launch
@@ -523,15 +548,7 @@ void row_tiling(int rows, int maxmt, int& mt, int& tiles) {
 // 16.5 -> 13.4 folded (5x2 -> 2x5), of 32x32x65 13.5 -> 6.2 and 11.8 -> 5.7,
 // of 128x128x257 65.8 -> 46.8 and 42.5 -> 32.7; 256x256x257 keeps 11x3 and 6x3.
 static void launch_tiling(int rows, int maxmt, bool folded, int cols, int& mt, int& tiles) {
-  static const int sms = [] {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
-      (void)cudaGetLastError();
-      n = 148;
-    }
-    return n;
-  }();
+  const int sms = sm_count();
   double best = 0.0;
   for (int p = maxmt, last = 0; p >= 1; --p) {
     int m = 0, t = 0;
@@ -679,11 +696,23 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
   int mt = op0.mt, tiles = op0.tiles;
   if ((op0.sym ? op0.pref_sym : op0.pref_dense) == 0)
     launch_tiling(op0.rows, op0.sym ? kMaxMtSym : kMaxMtDense, op0.sym, (2 * M + 127) / 128 * total, mt, tiles);
+  // The input comes by cp.async, never through the read-only path, so a launch
+  // whose epilogue reads only constant tables may be placed early; the others'
+  // operands (loaded ahead of the stores as read-only data) must be complete.
+  bool early = true;
+  for (int i = 0; i < nprob; ++i)
+    early = early && (probs[i].ep.mode == EPI_STORE || probs[i].ep.mode == EPI_RSCALE);
+  const dim3 grid(tiles, (2 * M + 127) / 128, total);
+  auto launch = [&](auto kernel, size_t smem) {
+    if (early)
+      launch_pdl(kernel, grid, kThreads, smem, s, grp[0], grp[1], grp[2]);
+    else
+      kernel<<<grid, kThreads, smem, s>>>(grp[0], grp[1], grp[2]);
+  };
   prof_begin(s, PC_GEMM, by, fl, xfl);
   if (op0.sym) {
     const bool split_in = op0.split == 2;
-    dim3 grid(tiles, (2 * M + 127) / 128, total);
-#define TG_SYM(MT, NP, SI) zgemm_sym_kernel<MT, NP, SI><<<grid, kThreads, sym_smem<MT>(), s>>>(grp[0], grp[1], grp[2])
+#define TG_SYM(MT, NP, SI) launch(zgemm_sym_kernel<MT, NP, SI>, sym_smem<MT>())
 #define TG_CASE(MT)                                              \
   case MT:                                                       \
     if (nprob == 1)                                              \
@@ -695,13 +724,12 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
 #undef TG_CASE
 #undef TG_SYM
   } else {
-    dim3 grid(tiles, (2 * M + 127) / 128, total);
 #define TG_CASE(MT)                                                                                       \
   case MT:                                                                                                \
     if (nprob == 1)                                                                                       \
-      zgemm_dense_kernel<MT, 1><<<grid, kThreads, dense_smem<MT>(), s>>>(grp[0], grp[1], grp[2]);        \
+      launch(zgemm_dense_kernel<MT, 1>, dense_smem<MT>());                                                \
     else                                                                                                  \
-      zgemm_dense_kernel<MT, kMaxGroup><<<grid, kThreads, dense_smem<MT>(), s>>>(grp[0], grp[1], grp[2]); \
+      launch(zgemm_dense_kernel<MT, kMaxGroup>, dense_smem<MT>());                                        \
     break;
     switch (mt) { TG_MT_LIST(TG_CASE) default: throw Error{TG_ERR_ARG, "zgemm > bad tiling"}; }
 #undef TG_CASE

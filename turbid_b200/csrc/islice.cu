@@ -170,6 +170,7 @@ struct SliceArgs {
 
 template <int S>
 __global__ void __launch_bounds__(kSliceThreads) k_slice_data(const SliceArgs a) {
+  pdl_begin();
   __shared__ double part_max[KP / 16][kSliceCols];
   const int lane = threadIdx.x & 31, kc = threadIdx.x >> 5;   // column in the block, K chunk
   const int pb = blockIdx.y;
@@ -280,6 +281,7 @@ struct IslArgs {
 // chains one after the other.
 template <int S>
 __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs args) {
+  pdl_begin();
   using Sh = IslShape<S>;
   constexpr int BN = Sh::BN;
   constexpr int kHalf = Sh::kTileA / 2;               // bytes of one half tile
@@ -687,9 +689,9 @@ void islice_group(const IsliceOp* const* ops, const double2* const* ins, double2
   const double fl = n * 4.0 * op0.nz * op0.nz * (double)M;
   prof_begin(s, PC_ISLICE, by, fl, fl);
   const int kchunks = (op0.nz - 2 + 31) / 32 * 2;   // 16-row K chunks in use
-  k_slice_data<5><<<dim3(op0.ntiles * (BM / kSliceCols), n), 32 * kchunks, 0, s>>>(sa);
+  launch_pdl(k_slice_data<5>, dim3(op0.ntiles * (BM / kSliceCols), n), 32 * kchunks, 0, s, sa);
   TG_LAUNCH_CHECK("k_slice_data");
-  k_islice_gemm<5><<<dim3(op0.ntiles, n), kGemmThreads, Sh::kSmem, s>>>(a);
+  launch_pdl(k_islice_gemm<5>, dim3(op0.ntiles, n), kGemmThreads, Sh::kSmem, s, a);
   prof_end(s);
   TG_LAUNCH_CHECK("k_islice_gemm");
 }

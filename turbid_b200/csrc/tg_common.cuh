@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <functional>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/turbid_gpu.h"
@@ -43,6 +44,52 @@ extern long long g_launches;   // kernel launches issued by this library (host t
       throw ::tg::Error{TG_ERR_CUDA, std::string(name) + " launch > " +         \
                                          cudaGetErrorString(e_)};               \
   } while (0)
+
+// ---------------------------------------------------------------------------
+// Early placement of the step's kernels (programmatic stream serialization).
+// Every kernel starts with pdl_begin().  A kernel launched with launch_pdl()
+// may have its blocks placed as soon as the last blocks of the kernel before
+// it in the stream run; they wait there, before their first memory access,
+// until that kernel has completed and its writes are visible, so the order of
+// memory accesses is that of plain launches and only launch latency is hidden.
+// Such a kernel is resident while its inputs are still being written, so it
+// must not read them through the read-only path (ld.global.nc: __ldg, const
+// __restrict__), which takes them as constant for the kernel's lifetime: the
+// transform, filter, slicing and product kernels read step data by plain
+// loads, cp.async or bulk copies; kernels that do not are launched plainly.
+//
+// Done only for grids of at most half the SMs, outside stream capture
+// (early_launch): two such kernels' blocks find SMs of their own.  Forward and
+// backward transform of 2 planes 64x64 FP32 16.4 -> 11.0 us, the per-stage
+// methods of 64x64x65 mixed 4.27 -> 3.61 ms for four steps.  Larger grids get
+// their waiting blocks piled on the SMs left free (33 planes 128x128 FP64
+// 19.5 -> 23.1 us, 195 planes 64x64 FP64 22.6 -> 31.1), and replayed graphs
+// gain nothing (laminar 32x32x65 step 0.25 ms with and without).
+// ---------------------------------------------------------------------------
+int sm_count();   // of the device current at the first call
+bool early_launch(dim3 grid, cudaStream_t s);
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = early_launch(grid, s) ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);   // checked by TG_LAUNCH_CHECK
+}
+#endif
 
 // ---------------------------------------------------------------------------
 // per-kernel-class timing with CUDA events (enabled by tg_profile_begin)
