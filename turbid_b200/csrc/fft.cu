@@ -719,31 +719,38 @@ __global__ void __launch_bounds__(NB * L / 16) by_p2_kernel(TransformDims d, con
 }
 
 // backward x pass, L = nx: two rows per complex FFT; Im of the kx = 0 coefficient ignored (c2r).
-// Backward x pass, first radix-16 pass straight from the row-major work
-// plane (FP32 layout [plane][y][kx], L >= 16): thread (b, j) forms Z[x] =
-// X1[x] + i X2[x] of row pair b at x = j + r * L/16 (X[L-k] = conj X[k]; zero
-// between the kept bands; Im of kx = 0 ignored), transforms the 16 values and
-// stores the pass's outputs in buf, so the packed rows are never staged in
-// shared memory before the pass.  One butterfly per thread (NB * L/16
-// threads); the caller synchronises and runs the passes of stride 16 on.
+// Backward x pass, first radix-16 pass straight from the work plane (L >= 16):
+// thread (b, j) forms Z[x] = X1[x] + i X2[x] of row pair b at x = j + r * L/16
+// (X[L-k] = conj X[k]; zero between the kept bands; Im of kx = 0 ignored),
+// transforms the 16 values and stores the pass's outputs in buf, so the packed
+// rows are never staged in shared memory before the pass.  Consecutive threads
+// take consecutive j where the plane is row-major ([y][kx], FP32) and
+// consecutive row pairs where it is column-major ([kx][y], FP64), along the
+// contiguous index.  One butterfly per thread (NB * L/16 threads); the caller
+// synchronises and runs the passes of stride 16 on.  FP64 up to L = 256
+// (backward transform, 20 M points: 32x32 484 -> 414 us, 64x64 160 -> 144,
+// 128x128 106 -> 100, 256x256 97 and 97); at 512 the staged rows stay (119
+// against 121 us).
 template <typename T, int L, int NB>
 __device__ __forceinline__ void bx_first_pass(cplx<T>* buf, const TransformDims& d,
                                               const cplx<T>* work, int plane, int y0) {
   using C = cplx<T>;
   constexpr int RS = P2<L>::RS;
   constexpr int nb = L / 16, nxh = L / 3 * 2 / 2 + 1;
-  const int b = threadIdx.x / nb, j = threadIdx.x - b * nb;
+  constexpr bool RM = P2Vec<T>::kBwdRowMajor;
+  const int b = RM ? threadIdx.x / nb : threadIdx.x % NB, j = RM ? threadIdx.x % nb : threadIdx.x / NB;
   const int ya = y0 + 2 * b, yb = ya + 1;
   const bool oka = ya < d.ny, okb = yb < d.ny;
   const C* src = work + (size_t)plane * nxh * d.ny;
-  const C* r1 = src + (size_t)(oka ? ya : 0) * nxh;
-  const C* r2 = src + (size_t)(okb ? yb : 0) * nxh;
+  const C* r1 = src + (size_t)(oka ? ya : 0) * (RM ? nxh : 1);
+  const C* r2 = src + (size_t)(okb ? yb : 0) * (RM ? nxh : 1);
+  const int st = RM ? 1 : d.ny;   // between two kx of a row
   C v[16];
 #pragma unroll
   for (int r = 0; r < 16; ++r) {
     const int x = j + r * nb;
     const bool lo = x < nxh, hi = x > L - nxh;
-    const int k = lo ? x : L - x;
+    const int k = (lo ? x : L - x) * st;
     C a = (oka && (lo || hi)) ? r1[k] : mkc<C>(0, 0);
     C c = (okb && (lo || hi)) ? r2[k] : mkc<C>(0, 0);
     if (x == 0) a.y = c.y = T(0);
@@ -844,7 +851,7 @@ __global__ void __launch_bounds__(NB * L / 16) bx_p2_kernel(TransformDims d, con
   const int plane = blockIdx.y;
   const int y0 = blockIdx.x * rows;
   T* dst = phys + (size_t)plane * d.ny * L;
-  if constexpr (L >= 32 && PV::kBwdRowMajor) {
+  if constexpr (L >= 32 && (PV::kBwdRowMajor || L <= 256)) {
     bx_first_pass<T, L, NB>(buf, d, work, plane, y0);
     __syncthreads();
     ip_passes<T, +1, L, NB, 16, NT, last_stride(L)>(buf, tw);
@@ -921,7 +928,7 @@ __global__ void __launch_bounds__(NB * L / 16, sizeof(T) == 4 ? 640 / (NB * L / 
   for (int i3 = 0; i3 < 3; ++i3) {
     const int j = yfirst && i3 < 2 ? 1 - i3 : i3;   // the order of the sum
     if (i3 > 0) __syncthreads();   // buf is refilled
-    if constexpr (L >= 16 && PV::kBwdRowMajor) {
+    if constexpr (L >= 16 && (PV::kBwdRowMajor || L <= 256)) {
       bx_first_pass<T, L, NB>(buf, d, work, (3 * c + j) * d.nz + z, y0);
       __syncthreads();
       ip_passes<T, +1, L, NB, 16>(buf, tw);
