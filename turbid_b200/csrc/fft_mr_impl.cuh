@@ -89,7 +89,6 @@ template <int L> struct Mr {
   static constexpr int NB = (n == 2 ? 128 : 256) / widest() < 1 ? 1 : (n == 2 ? 128 : 256) / widest();
   static constexpr int NT = (NB * widest() + 31) / 32 * 32;
   static constexpr int RS = (L + L / 16 + 1) | 1;                                  // padded row stride
-  static constexpr int PTS = (NB * L + NT - 1) / NT;                               // points per thread
   template <typename T> static constexpr size_t smem() { return (size_t)NB * RS * sizeof(cplx<T>); }
 };
 
@@ -412,55 +411,62 @@ __global__ void __launch_bounds__(Mr<L>::NT) mr_bx_kernel(int ny, const cplx<T>*
 
 // Backward x pass of ncomp groups of three gradient fields, each reduced to
 // the advection term (u + su) d/dx + (v + sv) d/dy + (w + sw) d/dz
-// (phase_carrier_flat.cc:786-797, phase_scalar_flat.cc:588-591): the sums of a
-// thread's points stay in its registers over the three gradients, whose
-// physical fields are never written.  grid: (row blocks x ncomp, nz),
-// component fastest, so that the velocity rows the ncomp CTAs share come from
-// DRAM once.
+// (phase_carrier_flat.cc:786-797, phase_scalar_flat.cc:588-591): a thread's
+// last butterfly covers the same points for the three gradients, so the sums
+// stay in its registers and the physical gradients are never written.  grid:
+// (row blocks x ncomp, nz), component fastest, so that the velocity rows the
+// ncomp CTAs share come from DRAM once.  The velocity values of a butterfly
+// are loaded side by side, rows beyond the last from the first row (not
+// stored): with a branch around each load the kernel waited for one load at a
+// time (144x144x145 class 0.380 -> 0.131 ms per step mixed, 0.680 -> 0.271
+// FP64).
 template <typename T, int L>
-__global__ void __launch_bounds__(Mr<L>::NT, sizeof(T) == 4 ? 640 / Mr<L>::NT : 1)
-    mr_adv_kernel(int nz, int ny, const cplx<T>* __restrict__ tw,
-                                                          const cplx<T>* work,
-                                                          const T* unl, T* out,
-                                                          int ncomp, double su, double sv, double sw) {
+__global__ void __launch_bounds__(Mr<L>::NT, sizeof(T) == 4 ? 512 / Mr<L>::NT : 1)
+    mr_adv_kernel(int nz, int ny, const cplx<T>* __restrict__ tw, const cplx<T>* work, const T* unl, T* out, int ncomp,
+                  double su, double sv, double sw) {
   pdl_begin();
   using C = cplx<T>;
   using P = Mr<L>;
-  constexpr int nxh = L / 3 * 2 / 2 + 1;
+  constexpr int nxh = L / 3 * 2 / 2 + 1, PS = P::n - 1, R = P::R(PS), nb = P::nb(PS);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int z = blockIdx.y, blk = blockIdx.x / ncomp, comp = blockIdx.x - blk * ncomp, y0 = blk * 2 * P::NB;
+  const int idx = threadIdx.x, j = idx % nb, b = idx / nb, ya = y0 + 2 * b;
+  const bool ok = b < P::NB, oka = ok && ya < ny, okb = ok && ya + 1 < ny;
   const size_t field = (size_t)nz * ny * L, off = ((size_t)z * ny + y0) * L;
-  C acc[P::PTS];   // of the point pairs e = threadIdx.x + i * NT: transform e / L, point e % L
+  const int oa = (oka ? 2 * b * L : 0) + j, ob = (okb ? (2 * b + 1) * L : 0) + j;
+  C acc[R];
 #pragma unroll
-  for (int i = 0; i < P::PTS; ++i) acc[i] = mkc<C>(0, 0);
+  for (int k = 0; k < R; ++k) acc[k] = mkc<C>(0, 0);
 #pragma unroll 1
   for (int i = 0; i < 3; ++i) {   // d/dy, d/dx, d/dz: u d/dx + v d/dy is one rounded product and one fused one
     const int g = i == 2 ? 2 : 1 - i;
     if (i > 0) __syncthreads();   // buf is refilled
     mr_bx_first<T, L>(buf, tw, work + (size_t)((3 * comp + g) * nz + z) * nxh * ny, ny, y0);
-    mr_passes<T, +1, L, 1, P::n>(buf, tw);
-    const T* uj = unl + g * field + off;
-    const T sh = (T)(g == 0 ? su : g == 1 ? sv : sw);
+    mr_passes<T, +1, L, 1, PS>(buf, tw);
+    if (ok) {
+      const T* uj = unl + g * field + off;
+      const T sh = (T)(g == 0 ? su : g == 1 ? sv : sw);
+      T ua[R], ub[R];
 #pragma unroll
-    for (int i = 0; i < P::PTS; ++i) {
-      const int e = threadIdx.x + i * P::NT, b = e / L, x = e % L, ya = y0 + 2 * b;
-      if (b < P::NB && ya < ny) {
-        const T* u = uj + 2 * b * L + x;
-        const C v = buf[b * P::RS + sp(x)];
-        acc[i].x += (u[0] + sh) * v.x;
-        if (ya + 1 < ny) acc[i].y += (u[L] + sh) * v.y;
+      for (int k = 0; k < R; ++k) {
+        ua[k] = uj[oa + k * nb];
+        ub[k] = uj[ob + k * nb];
+      }
+      C v[R];
+      mr_butterfly<T, +1, L, PS>(buf + b * P::RS, j, tw, v);
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        acc[k].x += (ua[k] + sh) * v[k].x;
+        acc[k].y += (ub[k] + sh) * v[k].y;
       }
     }
   }
   T* dst = out + comp * field + off;
 #pragma unroll
-  for (int i = 0; i < P::PTS; ++i) {
-    const int e = threadIdx.x + i * P::NT, b = e / L, x = e % L, ya = y0 + 2 * b;
-    if (b < P::NB && ya < ny) {
-      dst[2 * b * L + x] = acc[i].x;
-      if (ya + 1 < ny) dst[(2 * b + 1) * L + x] = acc[i].y;
-    }
+  for (int k = 0; k < R; ++k) {
+    if (oka) dst[oa + k * nb] = acc[k].x;
+    if (okb) dst[ob + k * nb] = acc[k].y;
   }
 }
 
