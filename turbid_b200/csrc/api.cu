@@ -1173,11 +1173,19 @@ static void run_ensemble(std::vector<Ctx*>& xs, int nsteps, int maxstep, double 
 // ---------------------------------------------------------------------------
 // The row tiling (m-tiles of 8 output rows per CTA) sets how often each CTA
 // column re-reads its input from L2 against how evenly the grid fills the
-// SMs; the best choice depends on Nz, M and the GPU.  The tuner times the
-// store-epilogue product of three components for each distinct tiling of the
-// dense and the folded kernel and keeps the fastest; the choice is cached in a
-// flat JSON object {"<Nx>x<Ny>x<Nz>:<precision>:sm<cc>x<SMs>": [dense, folded]}
-// of the two preferences (most m-tiles per CTA).
+// SMs; the best choice depends on Nz, M, the components of the launch and the
+// GPU.  By default it is chosen per launch (launch_tiling).  The tuner times the
+// store-epilogue product of one and of three components (a step's launches)
+// with that choice and with each distinct fixed tiling of the dense and the
+// folded kernel, and takes a fixed one for every launch only where it is faster
+// at both: the best fixed tiling at three components alone cost one component
+// of 128x128x257 93 -> 131 us per dense solve and 64 -> 85 split, of 64x64x129
+// 20 -> 32 and 14 -> 26.  The choice is cached in a flat JSON object
+// {"<Nx>x<Ny>x<Nz>:<precision>:sm<cc>x<SMs>:2": [dense, folded]} of the two
+// preferences (most m-tiles per CTA).  "Per launch" is written as the m-tiles
+// that choice takes at three components, and read from those or from 0.  The
+// last part of the key is the tuner's version: entries without one are the best
+// fixed tilings of a tuner that had no per-launch candidate.
 using TuneCache = std::map<std::string, std::pair<int, int>>;
 
 static std::string tune_key(const Ctx& x) {
@@ -1188,7 +1196,7 @@ static std::string tune_key(const Ctx& x) {
   TG_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
   TG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   char buf[128];
-  snprintf(buf, sizeof buf, "%dx%dx%d:%s:sm%d%dx%d", x.nx, x.ny, x.nz, x.mixed ? "mixed" : "fp64", major, minor,
+  snprintf(buf, sizeof buf, "%dx%dx%d:%s:sm%d%dx%d:2", x.nx, x.ny, x.nz, x.mixed ? "mixed" : "fp64", major, minor,
            sms);
   return buf;
 }
@@ -1230,7 +1238,7 @@ static void write_tune_cache(const char* path, const TuneCache& m) {
   }
 }
 
-// device milliseconds of one launch: the least mean over three runs of five
+// device milliseconds of one launch: the least mean over five runs of ten
 static float time_gemm(Ctx& x, const ZOperator& op, const double2* in, double2* out, int batch) {
   cudaEvent_t a = nullptr, b = nullptr;
   TG_CUDA(cudaEventCreate(&a));
@@ -1238,14 +1246,14 @@ static float time_gemm(Ctx& x, const ZOperator& op, const double2* in, double2* 
   float best = 1e30f;
   try {
     for (int w = 0; w < 2; ++w) gemm(x, op, in, x.S, out, x.S, batch, EpiParams());
-    for (int r = 0; r < 3; ++r) {
+    for (int r = 0; r < 5; ++r) {
       TG_CUDA(cudaEventRecord(a, x.s));
-      for (int i = 0; i < 5; ++i) gemm(x, op, in, x.S, out, x.S, batch, EpiParams());
+      for (int i = 0; i < 10; ++i) gemm(x, op, in, x.S, out, x.S, batch, EpiParams());
       TG_CUDA(cudaEventRecord(b, x.s));
       TG_CUDA(cudaEventSynchronize(b));
       float ms = 0.f;
       TG_CUDA(cudaEventElapsedTime(&ms, a, b));
-      best = std::min(best, ms / 5);
+      best = std::min(best, ms / 10);
     }
   } catch (...) {
     cudaEventDestroy(a);
@@ -1281,19 +1289,48 @@ static void apply_tiling(Ctx& x, int pd, int ps) {
   x.drop_graphs();   // the recorded launches carry the old grids
 }
 
+// The preference for one kernel: 0 (per launch), or the fixed tiling with the
+// least time of those that beat it at one and at three components.  2 % of the
+// time are left to the scatter of the timings.
+static int tune_kernel(Ctx& x, ZOperator op, int maxmt, int count, const double2* in, double2* out) {
+  auto set = [&](int p) { zop_set_tiling(op, op.sym ? 0 : p, op.sym ? p : 0); };
+  int mt0 = 0, tiles0 = 0;
+  launch_tiling(op.rows, op.sym, x.M, 3, mt0, tiles0);
+  set(0);
+  const float one = time_gemm(x, op, in, out, 1), three = time_gemm(x, op, in, out, 3);
+  float best = 0.98f * (one + three);
+  int pref = 0;
+  for (int p : tiling_candidates(op.rows, maxmt, count)) {
+    int mt = 0, tiles = 0;
+    row_tiling(op.rows, p, mt, tiles);
+    if (tiles == tiles0) continue;   // the per-launch choice at three components
+    set(p);
+    const float t1 = time_gemm(x, op, in, out, 1), t3 = time_gemm(x, op, in, out, 3);
+    if (t1 <= one && t3 <= three && t1 + t3 < best) best = t1 + t3, pref = p;
+  }
+  return pref;
+}
+
 static void autotune(Ctx& x, const char* cache_path, int* tiling) {
   int maxd = 0, maxs = 0;
   zop_tiling_limits(maxd, maxs);
   const std::string key = tune_key(x);
   TuneCache cache;
   if (cache_path) cache = read_tune_cache(cache_path);
+  // m-tiles x row tiles of the per-launch choice at three components
+  const int hr = (x.nz - 1) / 2 + 1;   // folded rows
+  int dmt = 0, dtiles = 0, smt = 0, stiles = 0;
+  launch_tiling(x.nz, false, x.M, 3, dmt, dtiles);
+  launch_tiling(hr, true, x.M, 3, smt, stiles);
   int pd = 0, ps = 0;
   auto hit = cache.find(key);
   if (hit != cache.end()) {
     pd = hit->second.first;
     ps = hit->second.second;
-    if (pd < 1 || pd > maxd || ps < 1 || ps > maxs)
+    if (pd < 0 || pd > maxd || ps < 0 || ps > maxs)
       throw Error{TG_ERR_ARG, "tg_autotune > cache entry " + key + " out of range"};
+    if (pd == dmt) pd = 0;
+    if (ps == smt) ps = 0;
   } else {
     TG_CUDA(cudaStreamSynchronize(x.s));
     if (x.s2) TG_CUDA(cudaStreamSynchronize(x.s2));
@@ -1313,26 +1350,14 @@ static void autotune(Ctx& x, const char* cache_path, int* tiling) {
         TG_CUDA(cudaMemcpyAsync(in, x.U, n * sizeof(double2), cudaMemcpyDeviceToDevice, x.s));
       else
         TG_CUDA(cudaMemsetAsync(in, 0x3f, n * sizeof(double2), x.s));   // finite non-zero values
-      // the dense kernel on the dense copy of D1, the folded kernel on D1 itself
-      ZOperator dense = x.opD1, folded = x.opD1;
+      // the dense kernel on the dense copy of D1, the folded kernel on D1
+      // itself (no folded operator on a grid of even Nz)
+      ZOperator dense = x.opD1;
       dense.sym = false;
       dense.split = 0;
-      float best = 1e30f;
-      for (int p : tiling_candidates(x.nz, maxd, 6)) {
-        zop_set_tiling(dense, p, 0);
-        const float ms = time_gemm(x, dense, in, out, 3);
-        if (ms < best) best = ms, pd = p;
-      }
-      best = 1e30f;
-      if (folded.sym) {
-        for (int p : tiling_candidates(folded.rows, maxs, 4)) {
-          zop_set_tiling(folded, 0, p);
-          const float ms = time_gemm(x, folded, in, out, 3);
-          if (ms < best) best = ms, ps = p;
-        }
-      } else {
-        ps = maxs;   // no folded operator on this grid (even Nz)
-      }
+      dense.rows = dense.n;
+      pd = tune_kernel(x, dense, maxd, 6, in, out);
+      if (x.opD1.sym) ps = tune_kernel(x, x.opD1, maxs, 4, in, out);
     } catch (...) {
       cudaFree(in);
       cudaFree(out);
@@ -1343,19 +1368,18 @@ static void autotune(Ctx& x, const char* cache_path, int* tiling) {
     TG_CUDA(cudaFree(out));
     g_prof = saved;
     if (cache_path) {
-      cache[key] = {pd, ps};
+      cache[key] = {pd ? pd : dmt, ps ? ps : smt};
       write_tune_cache(cache_path, cache);
     }
   }
   apply_tiling(x, pd, ps);
   if (tiling) {
-    int mt = 0, tiles = 0;
-    row_tiling(x.nz, pd, mt, tiles);
-    tiling[0] = mt;
-    tiling[1] = tiles;
-    row_tiling((x.nz - 1) / 2 + 1, ps, mt, tiles);
-    tiling[2] = mt;
-    tiling[3] = tiles;
+    if (pd) row_tiling(x.nz, pd, dmt, dtiles);
+    if (ps) row_tiling(hr, ps, smt, stiles);
+    tiling[0] = dmt;
+    tiling[1] = dtiles;
+    tiling[2] = smt;
+    tiling[3] = stiles;
   }
 }
 

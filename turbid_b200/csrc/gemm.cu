@@ -536,8 +536,8 @@ bool early_launch(dim3 grid, cudaStream_t s) {
   return st == cudaStreamCaptureStatusNone;
 }
 
-// Row tiling of one launch over `rows` rows and `cols` column tiles (128 reals,
-// all components): the tiling whose busiest SM has the least to do.  A CTA
+// Row tiling of one launch over `rows` rows and the column tiles (128 reals) of
+// `batch` components of M modes: the tiling whose busiest SM has the least to do.  A CTA
 // works at the FP64 tensor rate of its SM from two CTAs per SM on, so a launch
 // takes the m-tiles of the SM that gets the most CTAs, times a cost per m-tile
 // that falls with the tile height (the input columns are loaded once per CTA):
@@ -547,8 +547,8 @@ bool early_launch(dim3 grid, cudaStream_t s) {
 // of 128x128x129 20.6 -> 17.5 us dense (9x2 -> 4x5 m-tiles x row tiles) and
 // 16.5 -> 13.4 folded (5x2 -> 2x5), of 32x32x65 13.5 -> 6.2 and 11.8 -> 5.7,
 // of 128x128x257 65.8 -> 46.8 and 42.5 -> 32.7; 256x256x257 keeps 11x3 and 6x3.
-static void launch_tiling(int rows, int maxmt, bool folded, int cols, int& mt, int& tiles) {
-  const int sms = sm_count();
+void launch_tiling(int rows, bool folded, int M, int batch, int& mt, int& tiles) {
+  const int sms = sm_count(), maxmt = folded ? kMaxMtSym : kMaxMtDense, cols = (2 * M + 127) / 128 * batch;
   double best = 0.0;
   for (int p = maxmt, last = 0; p >= 1; --p) {
     int m = 0, t = 0;
@@ -692,10 +692,10 @@ static void zgemm_launch(const ZProblem* probs, int nprob, int M, cudaStream_t s
     grp[i] = grp[0];
     grp[i].batch = 0;
   }
-  // a tiling chosen by the autotuner holds for every launch of the operator
+  // a fixed tiling (a preference set) holds for every launch of the operator
   int mt = op0.mt, tiles = op0.tiles;
   if ((op0.sym ? op0.pref_sym : op0.pref_dense) == 0)
-    launch_tiling(op0.rows, op0.sym ? kMaxMtSym : kMaxMtDense, op0.sym, (2 * M + 127) / 128 * total, mt, tiles);
+    launch_tiling(op0.rows, op0.sym, M, total, mt, tiles);
   // The input comes by cp.async, never through the read-only path, so a launch
   // whose epilogue reads only constant tables may be placed early; the others'
   // operands (loaded ahead of the stores as read-only data) must be complete.

@@ -304,6 +304,7 @@ struct ZProblem {
 
 void zgemm_init();
 void row_tiling(int rows, int maxmt, int& mt, int& tiles);
+void launch_tiling(int rows, bool folded, int M, int batch, int& mt, int& tiles);
 void zop_build(ZOperator& op, const std::vector<double>& A, int n, bool allow_sym,
                const std::function<double*(size_t)>& alloc);
 // halves of one step of a split Helmholtz solve (split = 1: Einvs, 2: Es)

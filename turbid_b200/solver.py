@@ -132,9 +132,10 @@ class ChannelCase:
         check(self.lib.tg_set_zsolver(self.h, {"dmma": 0, "islice": 1}[solver]))
 
     def autotune(self, cache_path: Optional[str] = None) -> dict:
-        """Pick the z-operator GEMM row tiling for this grid and GPU (timed, or
-        read from the JSON cache at cache_path) and apply it; returns the
-        m-tiles per CTA and row tiles of the dense and the folded kernel."""
+        """Look for a fixed row tiling of the z-operator GEMMs that beats the
+        per-launch choice on this grid and GPU (timed, or read from the JSON
+        cache at cache_path) and apply it; returns the m-tiles per CTA and row
+        tiles of a three-component launch of the dense and the folded kernel."""
         t = (ctypes.c_int * 4)()
         path = None if cache_path is None else os.fsencode(cache_path)
         check(self.lib.tg_autotune(self.h, path, t))
