@@ -49,9 +49,13 @@ extern long long g_launches;   // kernel launches issued by this library (host t
 // Early placement of the step's kernels (programmatic stream serialization).
 // Every kernel starts with pdl_begin().  A kernel launched with launch_pdl()
 // may have its blocks placed as soon as the last blocks of the kernel before
-// it in the stream run; they wait there, before their first memory access,
-// until that kernel has completed and its writes are visible, so the order of
-// memory accesses is that of plain launches and only launch latency is hidden.
+// it in the stream have begun their own work; they wait there, before their
+// first memory access, until that kernel has completed and its writes are
+// visible, so the order of memory accesses is that of plain launches and only
+// launch latency is hidden.  A kernel releases its successor after its own wait:
+// released before it, the successor's successor could be placed as well, and so
+// on, a pile of waiting kernels holding SMs (64x64x65 mixed by the per-stage
+// methods 3.53 -> 3.48 ms for four steps, two planes unchanged).
 // Such a kernel is resident while its inputs are still being written, so it
 // must not read them through the read-only path (ld.global.nc: __ldg, const
 // __restrict__), which takes them as constant for the kernel's lifetime: the
@@ -59,20 +63,22 @@ extern long long g_launches;   // kernel launches issued by this library (host t
 // loads, cp.async or bulk copies; kernels that do not are launched plainly.
 //
 // Done only for grids of at most half the SMs, outside stream capture
-// (early_launch): two such kernels' blocks find SMs of their own.  Forward and
-// backward transform of 2 planes 64x64 FP32 16.4 -> 11.0 us, the per-stage
-// methods of 64x64x65 mixed 4.27 -> 3.61 ms for four steps.  Larger grids get
-// their waiting blocks piled on the SMs left free (33 planes 128x128 FP64
-// 19.5 -> 23.1 us, 195 planes 64x64 FP64 22.6 -> 31.1), and replayed graphs
-// gain nothing (laminar 32x32x65 step 0.25 ms with and without).
+// (early_launch): a kernel and the one that waits for it find SMs of their own,
+// so what other streams run beside them loses none.  Forward and backward
+// transform of 2 planes 64x64 FP32 16.4 -> 12.5 us, the per-stage methods of
+// 64x64x65 mixed 4.57 -> 3.48 ms for four steps.  Larger grids gain as well when
+// alone on the GPU (up to 592 blocks: 33 planes 128x128 FP64 18.5 -> 15.7 us, 195
+// planes 64x64 FP64 22.6 -> 19, 21 planes 250x90 FP64 26.6 -> 18.9); beside other
+// streams that is not measured, so they stay plain.  Replayed graphs gain
+// nothing (laminar 32x32x65 step 0.25 ms with and without).
 // ---------------------------------------------------------------------------
 int sm_count();   // of the device current at the first call
 bool early_launch(dim3 grid, cudaStream_t s);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <typename... P, typename... A>
