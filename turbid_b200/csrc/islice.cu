@@ -606,11 +606,7 @@ void islice_build(IsliceOp*& op, const std::vector<double>& A, int nrow, int nz,
   if (S != 5) throw Error{TG_ERR_ARG, "islice > only 5 slices are built"};
   if (nz < 3 || nz - 2 > KP) throw Error{TG_ERR_SHAPE, "islice > nz - 2 must be at most 256"};
   if ((size_t)A.size() != (size_t)nrow * nz) throw Error{TG_ERR_SHAPE, "islice > operator size"};
-  static bool smem_set = false;
-  if (!smem_set) {
-    islice_set_smem<5>();
-    smem_set = true;
-  }
+  islice_set_smem<5>();   // of the current context: a process may have several, on one GPU or more
   const int BN = IslShape<5>::BN, nchunks = (nrow + BN - 1) / BN;
   if (op && (op->nz != nz || op->nrow != nrow || op->ncol != 2 * M))
     throw Error{TG_ERR_SHAPE, "islice > rebuild with another shape"};
