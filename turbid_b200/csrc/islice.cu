@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs a
           "l"(dx), "l"(db), "r"(idesc), "r"(acc), "r"(elected));
     };
     int it = 0;
+    bool committed = false;
     for (int j = 0; j < nchunks && ok; ++j) {
       if (j > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_read, (j - 1) & 1, &s_err));
       asm volatile("tcgen05.fence::after_thread_sync;");
@@ -433,11 +434,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_islice_gemm(const IslArgs a
           "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
               ok ? bar_acc : bar_drain),
           "r"(elected));
+      committed = true;
     }
-    if (!ok) {   // the MMAs issued end before tensor and shared memory are released
-      s_err = 1;
-      if (it > 0) mbar_wait(bar_drain, 0);
-    }
+    if (!ok) s_err = 1;
+    // the MMAs issued end before tensor and shared memory are released, also
+    // where the epilogue gave up on the last chunk
+    if (committed) mbar_wait(ok ? bar_acc : bar_drain, ok ? (nchunks - 1) & 1 : 0);
   } else {   // ---- epilogue
     const int quarter = warp & 3, rgrp = warp >> 2;   // rows: 8-row groups rgrp, rgrp + 4, ...
     const int c = tile * BM + quarter * 32 + lane;
