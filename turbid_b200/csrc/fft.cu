@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(NB * L / 16) by_p2_kernel(TransformDims d, con
     for (int q = 0; q < 16; ++q) row[sp(16 * j + q)] = v[q];
     __syncthreads();
     ip_passes<T, +1, L, NB, 16>(buf, tw);
-  } else {
+  } else {   // 8 points: too few for a radix-16 first pass, the columns are staged
     constexpr int gap = L - nyc;  // FFT indices [nyc/2, L - nyc/2) carry no spectral row
     for (int idx = threadIdx.x; idx < NB * gap; idx += NT) {
       const int c = idx / gap, y = nyc / 2 + (idx - c * gap);

@@ -8,7 +8,12 @@ constexpr int kMrMaxLength = 512;
 
 // The lengths compiled: even, prime factors up to 7, not a power of two, at
 // least two radices (so that the last pass follows a first).  Odd lengths,
-// larger prime factors and lengths above 512 run the general kernels of fft.cu.
+// larger prime factors and lengths above 512 run the general kernels of fft.cu,
+// which are several times slower (forward and backward, 300 planes FP32: 225x225
+// 824 us, 224x224 95; 60 planes: 540x540 858, 500x500 170).  Nothing in the
+// passes needs an even length: each length adds ten kernels, about 230 KB of
+// library and some four seconds of compilation, and the 64 here are those that grids
+// of spectral cases use.
 constexpr bool mr_length(int L) {
   if (L < 18 || L > kMrMaxLength || L % 2 != 0 || (L & (L - 1)) == 0) return false;
   int n = L;

@@ -7,8 +7,12 @@
 // The radices of the general kernels (fours, a two, threes, fives, sevens),
 // in their order, are grouped into as few passes of at most 16 values as
 // possible (96 = (4 4)(2 3), 120 = (4 2)(3 5), 192 = (4 4)(4 3)), each
-// butterfly held in one thread's registers: the arithmetic is that of the
-// general kernels, value for value, without their passes through memory.  The
+// butterfly held in one thread's registers: the operations and their order are
+// those of the general kernels, without their passes through memory.  Which
+// products are fused into FMAs is left to the code generator (radix 2 apart,
+// cmul2), so equal bits are measured, not promised: with nvcc 12.9 every
+// compiled length gave the general kernels' values bit for bit, both precisions
+// and directions.  The
 // first pass takes its values straight from global memory, the last one hands
 // them on from its registers, and the passes between work in place on one
 // padded shared buffer: a two-pass length crosses shared memory once (twice
@@ -122,8 +126,8 @@ __device__ __forceinline__ void dft_e(cplx<T>* v, const cplx<T>* __restrict__ tw
   }
 }
 
-// a w, rounded as the general kernels' radix-2 pass rounds it (the code
-// generator fuses the other product of the imaginary part there)
+// a w, rounded as the general kernels' radix-2 pass rounds it (nvcc 12.9 fuses
+// the other product of the imaginary part there)
 __device__ __forceinline__ float2 cmul2(float2 a, float2 w) {
   return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.y, w.x, __fmul_rn(a.x, w.y)));
 }
@@ -135,7 +139,7 @@ __device__ __forceinline__ double2 cmul2(double2 a, double2 w) {
 // registers.  K values per group are already transformed: v[k * T + t], k < K,
 // t < T (T = values / K); NS: stride of the pass, jm: the butterfly's twiddle
 // index.  The operations and their order are those of one radix after the
-// other through memory, so the results do not depend on the grouping.
+// other through memory, whatever the grouping.
 template <typename T, int DIR, int L, int I, int END, int NS, int K, int N>
 __device__ __forceinline__ void mr_radices(cplx<T>* v, int jm, const cplx<T>* __restrict__ tw) {
   using C = cplx<T>;

@@ -26,9 +26,10 @@
 // Layouts: one K-major tile per 128 data columns and slice (the MMA's A
 // operand, M = 128 columns, K = 256 interior rows padded with zeros) and one
 // K-major tile per BN operator rows and slice (the B operand, N = BN), both
-// written in the canonical no-swizzle core-matrix order (8 rows x 16 bytes,
-// K chunks 128 bytes apart, 8-row groups 2048 bytes apart) so that each tile
-// is one contiguous bulk copy into shared memory.  The CTA keeps its 128
+// written in the 128-byte-swizzled order that the MMA reads (ksw_off: two
+// halves of 128 bytes of K one after the other, in each the 8-row atoms 1024
+// bytes apart), so that a half's rows in use are one contiguous bulk copy into
+// shared memory.  The CTA keeps its 128
 // columns' S data tiles in shared memory and walks the operator in chunks of
 // BN rows; one warp issues the bulk copies, one the MMAs, and sixteen read
 // each chunk's accumulators from tensor memory (thread = lane = data column),
